@@ -117,12 +117,21 @@ std::string device_name(int dev) {
 }
 }  // namespace
 
+// Name of device `dev`, queried once per process: cudaGetDeviceProperties takes ≈2.4 ms and, on a
+// host whose driver is busy, up to hundreds of ms, and every batch asks once per cell.  A failed
+// query is not kept.
+static std::string device_name_locked(int dev) {
+  auto it = g_dev_names.find(dev);
+  if (it != g_dev_names.end()) return it->second;
+  const std::string name = device_name(dev);
+  if (name != "unknown") g_dev_names[dev] = name;
+  return name;
+}
+
 static std::string current_device_name_locked() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return "unknown";
-  auto it = g_dev_names.find(dev);
-  if (it != g_dev_names.end()) return it->second;
-  return g_dev_names[dev] = device_name(dev);
+  return device_name_locked(dev);
 }
 
 TileChoice tiles_for(int Nx, int Ny) {
@@ -135,10 +144,9 @@ TileChoice tiles_for(int Nx, int Ny) {
 }
 
 bool tune_known(int dev, int Nx, int Ny) {
-  const std::string name = device_name(dev);
   std::lock_guard<std::mutex> lk(g_tune_mu);
   ensure_loaded_locked();
-  return g_tune.count(TuneKey{name, Nx, Ny}) > 0;
+  return g_tune.count(TuneKey{device_name_locked(dev), Nx, Ny}) > 0;
 }
 
 // Times the tile × wave variants (168 slots; each cluster apply once) of one FP32 M̂ application to `ncol` columns on `units`
