@@ -276,7 +276,7 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
   const int gstages = (int)std::max<size_t>(2, std::min<size_t>(8, (200 * 1024 - 128 - gred) / gstage));
   const size_t sm_gram = 128 + gstages * gstage + gred;
   const size_t sm_upd = UpdCfg<T>::smem;
-  const size_t sm_rr = 4 * (size_t)NMAX * NMAX * sizeof(double2);
+  const size_t sm_rr = rr_smem(nmax);
   OMB_CU(set_smem(k_gram<T>, sm_gram));
   auto update_kernel = Mmax <= 2 ? k_update<T, 2>
                        : Mmax <= 4 ? k_update<T, 4>
@@ -378,7 +378,7 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
                                                        d_err_.p, ctx_->wait_ns);
     if (!ok("k_gram", cudaGetLastError())) return e;
     k_rr<<<n, RR_NT, sm_rr, s>>>(d_state_ptrs_.p + a, d_gram_ptrs_.p + a, d_coef_ptrs_.p + a, d_coef32_ptrs_.p + a, n,
-                                 prm);
+                                 nmax, prm);
     if (!ok("k_rr", cudaGetLastError())) return e;
     update_kernel<<<grid_u, UpdCfg<T>::NT, sm_upd, s>>>(d_descs.p + a, preu, wpreu, n, par, prm.prec_diag,
                                                         d_err_.p, ctx_->wait_ns);

@@ -48,10 +48,99 @@ __global__ void k_live_prefix(TrackState* const* __restrict__ states, const long
   }
 }
 
+// The track's summed Gram matrices G = ZᴴZ and S = ZᴴAZ (upper triangles), scaled to unit
+// diagonal of G, and their reduction to the standard problem T = L⁻¹SL⁻ᴴ with G = LLᴴ.  Thread
+// (ty, tx) holds the elements (ty + 16a, tx + 16b) of G, S and Z in registers; step j eliminates
+// column j from all three at once (G ← its Schur complement, S ← E_j S E_jᴴ, Z ← Z E_jᴴ, so that Z
+// ends as L⁻ᴴ up to the pivots' roots): the only data exchanged are the three columns j, published
+// by their owners in a double-buffered shared copy, so a step is one barrier and the factorisation
+// and both triangular solves are n steps instead of 3n.  T (Hermitian) and Z go to shared memory.
+// Returns false when a pivot falls to the floor (near-dependent directions).
+struct RRCols { double2 g[2][NMAX], s[2][NMAX], z[2][NMAX]; };
+template <int TL>
+__device__ __forceinline__ bool rr_reduce(const double2* __restrict__ acc, int n, int ld, double drop, RRCols& col,
+                                          double* dsc, double2* T, double2* Z) {
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  double2 g[TL][TL], s[TL][TL], z[TL][TL];
+#pragma unroll
+  for (int a = 0; a < TL; ++a)
+#pragma unroll
+    for (int b = 0; b < TL; ++b) {
+      const int i = ty + 16 * a, k = tx + 16 * b;
+      g[a][b] = s[a][b] = z[a][b] = make_double2(0, 0);
+      if (i >= n || k >= n) continue;
+      const int lo = min(i, k), hi = max(i, k);
+      const double gi = acc[i * NMAX + i].x, gk = acc[k * NMAX + k].x;
+      const double di = gi > 0 && isfinite(gi) ? 1.0 / sqrt(gi) : 0.0, dk = gk > 0 && isfinite(gk) ? 1.0 / sqrt(gk) : 0.0;
+      const double2 vg = acc[lo * NMAX + hi], vs = acc[NMAX * NMAX + lo * NMAX + hi];
+      const double f = di * dk, sg = i < k ? f : (i > k ? -f : 0.0);
+      g[a][b] = make_double2(vg.x * f, vg.y * sg);
+      s[a][b] = make_double2(vs.x * f, vs.y * sg);
+      z[a][b].x = i == k ? 1.0 : 0.0;
+      if (i == k) dsc[i] = di;
+      if (k == 0) { col.g[0][i] = g[a][b]; col.s[0][i] = s[a][b]; col.z[0][i] = z[a][b]; }
+    }
+  __syncthreads();
+  for (int j = 0; j < n; ++j) {
+    const int cb = j & 1;
+    const double d = col.g[cb][j].x;
+    if (!(d > drop)) return false;  // the same value in every thread
+    const double inv = 1.0 / d;
+    const double2 sjj = col.s[cb][j];
+#pragma unroll
+    for (int b = 0; b < TL; ++b) {
+      const int k = tx + 16 * b;
+      if (k >= n) continue;
+      const double2 gk = col.g[cb][k], sk = col.s[cb][k];
+      const double2 lk = k > j ? make_double2(gk.x * inv, -gk.y * inv) : make_double2(0, 0);  // conj(l_kj)
+#pragma unroll
+      for (int a = 0; a < TL; ++a) {
+        const int i = ty + 16 * a;
+        if (i >= n) continue;
+        const double2 gi = col.g[cb][i], si = col.s[cb][i], zi = col.z[cb][i];
+        const double2 li = i > j ? make_double2(gi.x * inv, gi.y * inv) : make_double2(0, 0);
+        const double2 nl = make_double2(-lk.x, -lk.y), ni = make_double2(-li.x, -li.y);
+        if (i > j && k > j) g[a][b] = cmac(g[a][b], gi, nl);
+        // S_ik − l_i S_jk − conj(l_k)(S_ij − l_i S_jj)
+        s[a][b] = cmac(cmac(s[a][b], ni, make_double2(sk.x, -sk.y)), nl, cmac(si, ni, sjj));
+        z[a][b] = cmac(z[a][b], nl, zi);
+        if (k == j + 1) { col.g[cb ^ 1][i] = g[a][b]; col.s[cb ^ 1][i] = s[a][b]; col.z[cb ^ 1][i] = z[a][b]; }
+      }
+    }
+    __syncthreads();
+  }
+  // unit pivots: the diagonal of the final Schur complements is still in its owners' registers
+  double* piv = reinterpret_cast<double*>(col.g);
+#pragma unroll
+  for (int a = 0; a < TL; ++a) {
+    const int i = ty + 16 * a;
+    if (tx == (i & 15) && i < n) piv[i] = 1.0 / sqrt(g[a][a].x);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < TL; ++a)
+#pragma unroll
+    for (int b = 0; b < TL; ++b) {
+      const int i = ty + 16 * a, k = tx + 16 * b;
+      if (i >= n || k >= n) continue;
+      const double pk = piv[k], f = piv[i] * pk;
+      Z[i * ld + k] = make_double2(z[a][b].x * pk, z[a][b].y * pk);
+      if (i < k) continue;
+      const double2 t = make_double2(s[a][b].x * f, i == k ? 0.0 : s[a][b].y * f);
+      T[i * ld + k] = t;
+      T[k * ld + i] = make_double2(t.x, -t.y);
+    }
+  __syncthreads();
+  return true;
+}
+
+// One CTA per track: a latency-bound chain, so the time is what its barriers and dependent FP64
+// operations take.  The reduction is n one-barrier steps (rr_reduce), the eigenproblem FP32 Jacobi
+// sweeps refined to FP64 (eigh_refined), and L⁻ᴴ is applied as a matrix product.
 __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ states,
                                                double2* const* __restrict__ gram_accs,
                                                double2* const* __restrict__ coefs,
-                                               float2* const* __restrict__ coefs32, int ntracks,
+                                               float2* const* __restrict__ coefs32, int ntracks, int nmax,
                                                IterParams prm) {
   const int t = blockIdx.x;
   if (t >= ntracks) return;
@@ -60,135 +149,69 @@ __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ st
   const int M = s.M;
   const int n = M + s.nWa + s.nP;
   const double jtol2 = prm.jacobi_tol2;
-  constexpr int ld = NMAX;
+  const int ld = rr_ld(nmax);
+  const size_t mat = rr_mat(nmax);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* G = reinterpret_cast<double2*>(smem_raw);
-  double2* S = G + NMAX * NMAX;
-  double2* V = S + NMAX * NMAX;
-  double2* B = V + NMAX * NMAX;
+  double2* T = reinterpret_cast<double2*>(smem_raw);
+  double2* X = T + mat;
+  double2* W = X + mat;
+  double2* Y = W + mat;
+  double2* Z = Y + mat;
+  __shared__ RRCols cols;
   __shared__ RotIdx ri[NMAX];
   __shared__ double red[64];
   __shared__ int order[NMAX];
   __shared__ double dsc[NMAX];
   __shared__ double theta[NMAX];
+  __shared__ double lam[NMAX];
   __shared__ int keep[NMAX];
   __shared__ int rank;
   const int tid = threadIdx.x, nt = blockDim.x;
   double2* acc = gram_accs[t];
-  // 1. the summed Gram matrices (upper triangles), mirrored; then clear the accumulators
-  for (int e = tid; e < 2 * n * n; e += nt) {
-    const int which = e / (n * n), ab = e % (n * n), a = ab / n, b = ab % n;
-    if (a > b) continue;
-    double2 g = acc[which * NMAX * NMAX + a * NMAX + b];
-    double2* Mx = which ? S : G;
-    if (a == b) g.y = 0;
-    Mx[a * ld + b] = g;
-    Mx[b * ld + a] = make_double2(g.x, -g.y);
-  }
-  __syncthreads();
-  for (int e = tid; e < 2 * n * n; e += nt) {
-    const int which = e / (n * n), ab = e % (n * n), a = ab / n, b = ab % n;
-    if (a <= b) acc[which * NMAX * NMAX + a * NMAX + b] = make_double2(0, 0);
-  }
-  // 2. unit-diagonal scaling
-  for (int a = tid; a < n; a += nt) {
-    const double g = G[a * ld + a].x;
-    dsc[a] = (g > 0 && isfinite(g)) ? 1.0 / sqrt(g) : 0.0;
-  }
-  __syncthreads();
-  for (int e = tid; e < n * n; e += nt) {
-    const int a = e / n, b = e % n;
-    const double f = dsc[a] * dsc[b];
-    G[a * ld + b].x *= f; G[a * ld + b].y *= f;
-    S[a * ld + b].x *= f; S[a * ld + b].y *= f;
-    B[a * ld + b] = G[a * ld + b];  // the SVQB path needs it after the Cholesky attempt
-  }
-  __syncthreads();
-  // 3. Basis of the Gram metric.  Fast path: Cholesky Gs = L Lᴴ, then the projected
-  //    problem L⁻¹ Ss L⁻ᴴ u = λu and C = D L⁻ᴴ u.  When a pivot falls below the floor
-  //    (near-dependent directions) the SVQB path below drops them instead.
-  __shared__ int chol_ok;
-  if (tid == 0) chol_ok = 1;
-  __syncthreads();
-  for (int j = 0; j < n; ++j) {
-    const double piv = G[j * ld + j].x;
-    if (!(piv > prm.gram_drop)) { chol_ok = 0; break; }  // uniform across the block
-    const double ljj = sqrt(piv);
-    for (int i = j + 1 + tid; i < n; i += nt) {
-      const double2 g = G[i * ld + j];
-      G[i * ld + j] = make_double2(g.x / ljj, g.y / ljj);
-    }
-    __syncthreads();
-    if (tid == 0) G[j * ld + j] = make_double2(ljj, 0.0);
-    const int w = n - j - 1;
-    for (int e = tid; e < w * w; e += nt) {
-      const int i = j + 1 + e / w, k = j + 1 + e % w;
-      if (k <= i) {
-        const double2 li = G[i * ld + j], lk = G[k * ld + j];
-        G[i * ld + k].x -= li.x * lk.x + li.y * lk.y;  // L_ij·conj(L_kj)
-        G[i * ld + k].y -= li.y * lk.x - li.x * lk.y;
-      }
-    }
-    __syncthreads();
-  }
-  __syncthreads();
-  int r;
-  double2* Ev;  // eigenvectors of the projected problem (columns), n_eff × n_eff
-  double2* Av;  // the projected matrix, eigenvalues on its diagonal after Jacobi
+  const bool chol_ok = n <= 16   ? rr_reduce<1>(acc, n, ld, prm.gram_drop, cols, dsc, T, Z)
+                       : n <= 32 ? rr_reduce<2>(acc, n, ld, prm.gram_drop, cols, dsc, T, Z)
+                                 : rr_reduce<3>(acc, n, ld, prm.gram_drop, cols, dsc, T, Z);
+  int r = n;
+  const double2* Ev;  // eigenvectors of the projected problem (columns)
+  double2* G = T;     // SVQB path: scaled Gram matrix, then the projected one
+  double2* B = W;     // SVQB path: the kept basis
   if (chol_ok) {
-    r = n;
-    // V ← L⁻¹ Ss (column-parallel forward substitution)
-    for (int c = tid; c < n; c += nt) {
-      for (int i = 0; i < n; ++i) {
-        double2 t = S[i * ld + c];
-        for (int k = 0; k < i; ++k) {
-          const double2 l = G[i * ld + k], v = V[k * ld + c];
-          t.x -= l.x * v.x - l.y * v.y;
-          t.y -= l.x * v.y + l.y * v.x;
-        }
-        const double d = G[i * ld + i].x;
-        V[i * ld + c] = make_double2(t.x / d, t.y / d);
-      }
+    // the accumulators are read: clear them for the next iteration
+    for (int a = tid / 16; a < n; a += nt / 16)
+      for (int b = a + tid % 16; b < n; b += 16)
+        acc[a * NMAX + b] = acc[NMAX * NMAX + a * NMAX + b] = make_double2(0, 0);
+    const double tol_e = 0.03 * sqrt(sqrt(jtol2));  // the last step leaves ‖E‖² ≲ 1e-3·√jtol2
+    Ev = n <= 16   ? eigh_refined<1>(T, X, Y, W, n, M, ld, lam, red, order, tol_e)
+         : n <= 32 ? eigh_refined<2>(T, X, Y, W, n, M, ld, lam, red, order, tol_e)
+                   : eigh_refined<3>(T, X, Y, W, n, M, ld, lam, red, order, tol_e);
+    if (!Ev) {
+      __syncthreads();
+      jacobi_eigh(T, X, n, ld, W, ri, red, jtol2);
+      for (int i = tid; i < n; i += nt) lam[i] = T[i * ld + i].x;
+      Ev = X;
     }
-    __syncthreads();
-    // B ← L⁻¹ Vᴴ = L⁻¹ Ss L⁻ᴴ
-    for (int c = tid; c < n; c += nt) {
-      for (int i = 0; i < n; ++i) {
-        const double2 vc = V[c * ld + i];
-        double2 t = make_double2(vc.x, -vc.y);
-        for (int k = 0; k < i; ++k) {
-          const double2 l = G[i * ld + k], v = B[k * ld + c];
-          t.x -= l.x * v.x - l.y * v.y;
-          t.y -= l.x * v.y + l.y * v.x;
-        }
-        const double d = G[i * ld + i].x;
-        B[i * ld + c] = make_double2(t.x / d, t.y / d);
-      }
-    }
-    __syncthreads();
-    for (int e = tid; e < n * n; e += nt) {  // Hermitian part
-      const int i = e / n, j = e % n;
-      if (i < j) {
-        const double2 x = B[i * ld + j], y = B[j * ld + i];
-        const double2 h = make_double2(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
-        B[i * ld + j] = h;
-        B[j * ld + i] = make_double2(h.x, -h.y);
-      } else if (i == j) {
-        B[i * ld + i].y = 0;
-      }
-    }
-    __syncthreads();
-    jacobi_eigh(B, V, r, ld, S, ri, red, jtol2);  // S is free once B = L⁻¹ S L⁻ᴴ
-    Ev = V;
-    Av = B;
   } else {
-    // SVQB: restore the scaled Gram matrix (the Cholesky attempt overwrote it)
-    for (int e = tid; e < n * n; e += nt) {
-      const int a = e / n, b = e % n;
-      G[a * ld + b] = B[a * ld + b];
+    // SVQB on the scaled Gram matrix
+    double2* S = X;
+    double2* V = Y;
+    __syncthreads();
+    for (int e = tid; e < 2 * n * n; e += nt) {
+      const int which = e / (n * n), ab = e % (n * n), a = ab / n, b = ab % n;
+      if (a > b) continue;
+      const double f = dsc[a] * dsc[b];
+      double2 g = acc[which * NMAX * NMAX + a * NMAX + b];
+      g.x *= f;
+      g.y *= a == b ? 0.0 : f;
+      double2* Mx = which ? S : G;
+      Mx[a * ld + b] = g;
+      Mx[b * ld + a] = make_double2(g.x, -g.y);
     }
     __syncthreads();
-    jacobi_eigh(G, V, n, ld, B, ri, red, jtol2);  // B's copy of G is back in G
+    for (int e = tid; e < 2 * n * n; e += nt) {
+      const int which = e / (n * n), ab = e % (n * n), a = ab / n, b = ab % n;
+      if (a <= b) acc[which * NMAX * NMAX + a * NMAX + b] = make_double2(0, 0);
+    }
+    jacobi_eigh(G, V, n, ld, B, ri, red, jtol2);
     if (tid == 0) {
       double tmax = 0;
       for (int i = 0; i < n; ++i) { theta[i] = G[i * ld + i].x; tmax = fmax(tmax, theta[i]); }
@@ -238,57 +261,42 @@ __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ st
     }
     __syncthreads();
     jacobi_eigh(G, V, r, ld, S, ri, red, jtol2);  // S is folded into G = Bᴴ S B
+    for (int i = tid; i < r; i += nt) lam[i] = G[i * ld + i].x;
     Ev = V;
-    Av = G;
   }
-  sort_diag(Av, r, ld, order);
-  // 5. coefficients of the new X in the Z columns, Ritz values
+  __syncthreads();
+  // ascending Ritz values
+  if (tid < r) {
+    const double d = lam[tid];
+    int at = 0;
+    for (int j = 0; j < r; ++j) at += lam[j] < d || (lam[j] == d && j < tid);
+    order[at] = tid;
+  }
+  __syncthreads();
+  // coefficients of the new X in the Z columns (D L⁻ᴴ U, or D B U), and of the new P for the active
+  // columns: the W and P parts of the Ritz vectors
   double2* coef = coefs[t];
   float2* coef32 = coefs32[t];
-  if (chol_ok) {
-    // C = D L⁻ᴴ U[:, order[:M]] (column-parallel back substitution; S is free scratch)
-    for (int m = tid; m < M; m += nt) {
-      const int um = order[m];
-      for (int i = n - 1; i >= 0; --i) {
-        double2 y = Ev[i * ld + um];
-        for (int k = i + 1; k < n; ++k) {
-          const double2 l = G[k * ld + i], v = S[k * ld + m];  // conj(L_ki)·y_k
-          y.x -= l.x * v.x + l.y * v.y;
-          y.y -= l.x * v.y - l.y * v.x;
-        }
-        const double d = G[i * ld + i].x;
-        S[i * ld + m] = make_double2(y.x / d, y.y / d);
-      }
-      for (int i = 0; i < n; ++i) {
-        const double2 y = S[i * ld + m];
-        coef[i * MMAX + m] = make_double2(y.x * dsc[i], y.y * dsc[i]);
-        coef32[i * MMAX + m] = make_float2((float)(y.x * dsc[i]), (float)(y.y * dsc[i]));
-      }
-    }
-  } else {
-    for (int e = tid; e < n * M; e += nt) {
-      const int l = e / M, m = e % M;
-      const int um = order[m];
-      double2 acc = make_double2(0, 0);
-      for (int j = 0; j < r; ++j) {
-        const double2 a = B[l * ld + j], b = Ev[j * ld + um];
-        acc.x += a.x * b.x - a.y * b.y;
-        acc.y += a.x * b.y + a.y * b.x;
-      }
-      coef[l * MMAX + m] = make_double2(acc.x * dsc[l], acc.y * dsc[l]);
-      coef32[l * MMAX + m] = make_float2((float)(acc.x * dsc[l]), (float)(acc.y * dsc[l]));
-    }
-  }
-  for (int m = tid; m < M; m += nt) s.lam[m] = Av[order[m] * ld + order[m]].x;
-  __syncthreads();
-  // 6. P coefficients for the active columns: the W and P parts of the Ritz vectors
+  const double2* Bz = chol_ok ? Z : B;
   const int nPn = (s.nWa + s.nP > 0) ? (M - s.nlocked) : 0;
-  for (int e = tid; e < n * nPn; e += nt) {
-    const int l = e / nPn, mp = e % nPn;
-    const double2 c = (l < M) ? make_double2(0, 0) : coef[l * MMAX + (s.nlocked + mp)];
-    coef[NMAX * MMAX + l * MMAX + mp] = c;
-    coef32[NMAX * MMAX + l * MMAX + mp] = make_float2((float)c.x, (float)c.y);
+  for (int e = tid; e < n * MMAX; e += nt) {
+    const int l = e / MMAX, m = e % MMAX;
+    if (m >= M) continue;
+    const int um = order[m];
+    double2 c = make_double2(0, 0);
+    for (int j = chol_ok ? l : 0; j < r; ++j) c = cmac(c, Bz[l * ld + j], Ev[j * ld + um]);
+    c.x *= dsc[l];
+    c.y *= dsc[l];
+    coef[l * MMAX + m] = c;
+    coef32[l * MMAX + m] = make_float2((float)c.x, (float)c.y);
+    const int mp = m - s.nlocked;
+    if (mp >= 0 && mp < nPn) {
+      if (l < M) c = make_double2(0, 0);
+      coef[NMAX * MMAX + l * MMAX + mp] = c;
+      coef32[NMAX * MMAX + l * MMAX + mp] = make_float2((float)c.x, (float)c.y);
+    }
   }
+  for (int m = tid; m < M; m += nt) s.lam[m] = lam[order[m]];
   if (tid == 0) { s.nP_next = nPn; s.rr_n = n; s.rr_rank = r; }
 }
 

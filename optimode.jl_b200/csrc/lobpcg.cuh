@@ -32,7 +32,7 @@ namespace omb {
 constexpr int MMAX = 12;         // block columns per track
 constexpr int NMAX = 3 * MMAX;   // Rayleigh–Ritz basis size
 constexpr int LANES = 2;         // track lanes (streams) of an engine's iteration graph
-constexpr int RR_NT = 128;
+constexpr int RR_NT = EIG_NT;
 
 enum TrackStatus : int {
   TS_RUNNING = 0, TS_CONVERGED = 1, TS_MAXITER = 2, TS_ORTHO = 3, TS_NAN = 4, TS_PHASE_DONE = 5,
@@ -655,12 +655,18 @@ __global__ void __launch_bounds__(UpdCfg<T>::NT, 1)
 
 // ---------------------------------------------------------------------------------
 // Rayleigh–Ritz: one CTA per track.  Reads the track's Gram accumulators (and clears
-// them for the next iteration); writes C, CP in FP64 and in FP32 (coef32).
+// them for the next iteration); writes C, CP in FP64 and in FP32 (coef32).  nmax: the largest basis
+// of the launch (it sizes the shared matrices).
 __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ states,
                                                double2* const* __restrict__ gram_accs,
                                                double2* const* __restrict__ coefs,
-                                               float2* const* __restrict__ coefs32, int ntracks,
+                                               float2* const* __restrict__ coefs32, int ntracks, int nmax,
                                                IterParams prm);
+// k_rr's shared matrices for bases of up to nmax columns: five of rr_mat elements, rows of an odd
+// number of double2 (column reads then hit distinct banks)
+__host__ __device__ constexpr int rr_ld(int nmax) { return ((nmax + 1) / 2 * 2) | 1; }
+__host__ __device__ constexpr size_t rr_mat(int nmax) { return (size_t)((nmax + 1) / 2 * 2) * rr_ld(nmax); }
+__host__ __device__ constexpr size_t rr_smem(int nmax) { return 5 * rr_mat(nmax) * sizeof(double2); }
 
 // ---------------------------------------------------------------------------------
 // Control (after the update; one warp per track) and Newton (after the HMkH pass; one

@@ -205,3 +205,19 @@ def test_uneven_batch(omb):
             assert np.all(i["status"] == 0)
             assert np.allclose(km, ref, rtol=1e-9)
             assert len(kv) == pr["nev"] and all(v.shape == (2 * pr["grid"].N,) for v in kv)
+
+
+@pytest.mark.parametrize("nev", [1, 2, 4, 5, 7, 10, 11])
+def test_rayleigh_ritz_block_sizes(omb, case, nev):
+    """Blocks of nev + 1 columns, so Rayleigh–Ritz bases of up to 6, 9, 15, 18, 24, 33 and 36: one,
+    two and three 16-wide tiles per dimension of k_rr, even and odd sizes, and the largest.
+    FP64 at 1e-10, so eigenvalue errors are ≈ residual²/gap: rtol 1e-9 as for the other solves."""
+    grid, ei, _, _ = case
+    g = omb.Grid(6.0, 4.0, 24, 16)
+    k0 = O.k_guess(OMEGA0, ei)
+    ref, _, _ = O.solve_omega2(k0, ei, grid, nev=nev + 2, tol=1e-9, maxiter=600)
+    ev, evecs, info = omb.solve_omega2(k0, ei, g, omb.B200Solver(precision="fp64"), nev=nev, tol=1e-10, return_info=True)
+    assert np.all(info["status"] == 0)
+    assert np.allclose(ev, ref[:nev], rtol=1e-9, atol=0)
+    V = np.stack(evecs, axis=1)
+    assert np.allclose(V.conj().T @ V, np.eye(nev), atol=1e-10)
