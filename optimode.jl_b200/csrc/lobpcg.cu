@@ -56,7 +56,7 @@ __global__ void k_live_prefix(TrackState* const* __restrict__ states, const long
 // by their owners in a double-buffered shared copy, so a step is one barrier and the factorisation
 // and both triangular solves are n steps instead of 3n.  T (Hermitian) and Z go to shared memory.
 // Returns false when a pivot falls to the floor (near-dependent directions).
-struct RRCols { double2 g[2][NMAX], s[2][NMAX], z[2][NMAX]; };
+struct RRCols { double2 g[2][NMAX], s[2][NMAX], z[2][NMAX]; double d[2][NMAX]; };
 template <int TL>
 __device__ __forceinline__ bool rr_reduce(const double2* __restrict__ acc, int n, int ld, double drop, RRCols& col,
                                           double* dsc, double2* T, double2* Z) {
@@ -71,42 +71,50 @@ __device__ __forceinline__ bool rr_reduce(const double2* __restrict__ acc, int n
       if (i >= n || k >= n) continue;
       const int lo = min(i, k), hi = max(i, k);
       const double gi = acc[i * NMAX + i].x, gk = acc[k * NMAX + k].x;
-      const double di = gi > 0 && isfinite(gi) ? 1.0 / sqrt(gi) : 0.0, dk = gk > 0 && isfinite(gk) ? 1.0 / sqrt(gk) : 0.0;
+      const double di = gi > 0 && isfinite(gi) ? rsqrt(gi) : 0.0, dk = gk > 0 && isfinite(gk) ? rsqrt(gk) : 0.0;
       const double2 vg = acc[lo * NMAX + hi], vs = acc[NMAX * NMAX + lo * NMAX + hi];
       const double f = di * dk, sg = i < k ? f : (i > k ? -f : 0.0);
       g[a][b] = make_double2(vg.x * f, vg.y * sg);
       s[a][b] = make_double2(vs.x * f, vs.y * sg);
       z[a][b].x = i == k ? 1.0 : 0.0;
-      if (i == k) dsc[i] = di;
+      if (i == k) { dsc[i] = di; col.d[0][i] = g[a][b].x; }
       if (k == 0) { col.g[0][i] = g[a][b]; col.s[0][i] = s[a][b]; col.z[0][i] = z[a][b]; }
     }
   __syncthreads();
+  // the pivot of step j + 1 and its reciprocal are formed during step j, in every thread, from column
+  // j and the published diagonal, so the reciprocal is off the chain of the updates
+  double d = col.d[0][0], inv = 1.0 / d;
   for (int j = 0; j < n; ++j) {
     const int cb = j & 1;
-    const double d = col.g[cb][j].x;
     if (!(d > drop)) return false;  // the same value in every thread
-    const double inv = 1.0 / d;
+    const int jn = min(j + 1, n - 1);
+    const double2 gn = col.g[cb][jn];
+    const double dn = fma(-(gn.x * gn.x + gn.y * gn.y), inv, col.d[cb][jn]);
+    const double invn = 1.0 / dn;
     const double2 sjj = col.s[cb][j];
 #pragma unroll
     for (int b = 0; b < TL; ++b) {
-      const int k = tx + 16 * b;
-      if (k >= n) continue;
-      const double2 gk = col.g[cb][k], sk = col.s[cb][k];
-      const double2 lk = k > j ? make_double2(gk.x * inv, -gk.y * inv) : make_double2(0, 0);  // conj(l_kj)
+      const int k = tx + 16 * b, kc = min(k, n - 1);  // (threads outside the matrix repeat an edge)
+      const double2 gk = col.g[cb][kc], sk = col.s[cb][kc];
+      const double invk = k > j ? inv : 0.0;  // l is zero at and before the pivot
+      const double2 nl = make_double2(-gk.x * invk, gk.y * invk);  // −conj(l_kj)
 #pragma unroll
       for (int a = 0; a < TL; ++a) {
-        const int i = ty + 16 * a;
-        if (i >= n) continue;
-        const double2 gi = col.g[cb][i], si = col.s[cb][i], zi = col.z[cb][i];
-        const double2 li = i > j ? make_double2(gi.x * inv, gi.y * inv) : make_double2(0, 0);
-        const double2 nl = make_double2(-lk.x, -lk.y), ni = make_double2(-li.x, -li.y);
-        if (i > j && k > j) g[a][b] = cmac(g[a][b], gi, nl);
+        const int i = ty + 16 * a, ic = min(i, n - 1);
+        const double2 gi = col.g[cb][ic], si = col.s[cb][ic], zi = col.z[cb][ic];
+        const double invi = i > j ? inv : 0.0;
+        const double2 ni = make_double2(-gi.x * invi, -gi.y * invi);  // −l_ij
+        const double2 gm = i > j ? gi : make_double2(0, 0);
+        g[a][b] = cmac(g[a][b], gm, nl);
         // S_ik − l_i S_jk − conj(l_k)(S_ij − l_i S_jj)
         s[a][b] = cmac(cmac(s[a][b], ni, make_double2(sk.x, -sk.y)), nl, cmac(si, ni, sjj));
         z[a][b] = cmac(z[a][b], nl, zi);
-        if (k == j + 1) { col.g[cb ^ 1][i] = g[a][b]; col.s[cb ^ 1][i] = s[a][b]; col.z[cb ^ 1][i] = z[a][b]; }
+        if (k == j + 1 && i < n) { col.g[cb ^ 1][i] = g[a][b]; col.s[cb ^ 1][i] = s[a][b]; col.z[cb ^ 1][i] = z[a][b]; }
+        if (i == k && i < n) col.d[cb ^ 1][i] = g[a][b].x;
       }
     }
+    d = dn;
+    inv = invn;
     __syncthreads();
   }
   // unit pivots: the diagonal of the final Schur complements is still in its owners' registers
@@ -114,7 +122,7 @@ __device__ __forceinline__ bool rr_reduce(const double2* __restrict__ acc, int n
 #pragma unroll
   for (int a = 0; a < TL; ++a) {
     const int i = ty + 16 * a;
-    if (tx == (i & 15) && i < n) piv[i] = 1.0 / sqrt(g[a][a].x);
+    if (tx == (i & 15) && i < n) piv[i] = rsqrt(g[a][a].x);
   }
   __syncthreads();
 #pragma unroll
@@ -150,9 +158,8 @@ __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ st
   const int n = M + s.nWa + s.nP;
   const double jtol2 = prm.jacobi_tol2;
   const int ld = rr_ld(nmax);
-  const size_t mat = rr_mat(nmax);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* T = reinterpret_cast<double2*>(smem_raw);
+  const int mat = (int)rr_mat(nmax);
+  double2* T = reinterpret_cast<double2*>(rr_smem_raw);
   double2* X = T + mat;
   double2* W = X + mat;
   double2* Y = W + mat;
@@ -160,6 +167,8 @@ __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ st
   __shared__ RRCols cols;
   __shared__ RotIdx ri[NMAX];
   __shared__ double red[64];
+  __shared__ float redf[EIG_NT / 32];
+  __shared__ float4 rots[NMAX];
   __shared__ int order[NMAX];
   __shared__ double dsc[NMAX];
   __shared__ double theta[NMAX];
@@ -181,10 +190,11 @@ __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ st
       for (int b = a + tid % 16; b < n; b += 16)
         acc[a * NMAX + b] = acc[NMAX * NMAX + a * NMAX + b] = make_double2(0, 0);
     const double tol_e = 0.03 * sqrt(sqrt(jtol2));  // the last step leaves ‖E‖² ≲ 1e-3·√jtol2
-    Ev = n <= 16   ? eigh_refined<1>(T, X, Y, W, n, M, ld, lam, red, order, tol_e)
-         : n <= 32 ? eigh_refined<2>(T, X, Y, W, n, M, ld, lam, red, order, tol_e)
-                   : eigh_refined<3>(T, X, Y, W, n, M, ld, lam, red, order, tol_e);
-    if (!Ev) {
+    const int at = n <= 16   ? eigh_refined<1>(0, mat, 3 * mat, 2 * mat, n, M, ld, lam, redf, rots, order, tol_e)
+                   : n <= 32 ? eigh_refined<2>(0, mat, 3 * mat, 2 * mat, n, M, ld, lam, redf, rots, order, tol_e)
+                             : eigh_refined<3>(0, mat, 3 * mat, 2 * mat, n, M, ld, lam, redf, rots, order, tol_e);
+    Ev = T + at;
+    if (at < 0) {
       __syncthreads();
       jacobi_eigh(T, X, n, ld, W, ri, red, jtol2);
       for (int i = tid; i < n; i += nt) lam[i] = T[i * ld + i].x;

@@ -141,7 +141,7 @@ __device__ inline void jacobi_eigh(double2* A, double2* V, int n, int ld, double
 //
 // A round of the FP64 Jacobi above is a chain of dependent FP64 operations (three reciprocal
 // square roots, a reciprocal, two barriers; ≈2.5 K cycles at n = 15), and a matrix needs 6–8
-// sweeps of n − 1 rounds.  The sweeps below run on an FP32 copy (one barrier and ≈300 cycles a
+// sweeps of n − 1 rounds.  The sweeps below run on an FP32 copy (≈470 cycles a
 // round), and their eigenvectors are then brought to FP64 by the quadratically convergent
 // refinement of T. Ogita and K. Aishima ("Iterative refinement for symmetric eigenvalue
 // decomposition", Japan J. Indust. Appl. Math. 35, 2018), whose steps are three small matrix
@@ -155,103 +155,161 @@ constexpr int EIG_NT = 256;          // threads: a 16×16 map over matrix elemen
 constexpr float JAC32_ANGLE2 = 1e-6f, JAC32_NOISE2 = 2e-13f;
 constexpr double E_MAX = 0.1;
 
-__device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+// acc + conj(a)·b as a chain of two FMAs per half (like cmac)
+__device__ __forceinline__ double2 cmacc(double2 c, double2 a, double2 b) {
+  return make_double2(fma(a.y, b.y, fma(a.x, b.x, c.x)), fma(-a.y, b.x, fma(a.x, b.y, c.y)));
 }
-struct Rot32 { float c, s, er, ei; };  // rows: p ← c p − s e q, q ← s p + c e q; columns with ē
+// c·a + w·b (c real)
+__device__ __forceinline__ float2 rotf(float c, float2 a, float2 w, float2 b) {
+  return make_float2(fmaf(-w.y, b.y, fmaf(w.x, b.x, c * a.x)), fmaf(w.y, b.x, fmaf(w.x, b.y, c * a.y)));
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// Shared-memory accesses by 32-bit address.
+__device__ __forceinline__ float lds1(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float2 lds2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts2(uint32_t a, float2 v) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void sts4(uint32_t a, float4 v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+// rows: p ← c p − w q, q ← w̄ p + c q;  columns: p ← c p − w̄ q, q ← w p + c q
+struct Rot32 { float c; float2 w; };
 
-// The rotation that annihilates A_pq (identity when it is below the FP32 noise of a unit-norm
-// matrix); `big` reports a rotation that another sweep has to follow.
+// The rotation that annihilates A_pq of a unit-norm matrix: with d = A_qq − A_pp and
+// h = √(d² + 4|A_pq|²), c² = (1 + |d|/h)/2 and w = sign(d)·A_pq/(h c) — two reciprocal square roots in
+// sequence and no branch, so that the two rotations a thread needs overlap (1e-9 added to |d| makes
+// equal entries with A_pq = 0 the identity).  `big` reports one that another sweep has to follow.
 __device__ __forceinline__ Rot32 rot32(float2 apq, float app, float aqq, bool& big) {
-  const float g2 = apq.x * apq.x + apq.y * apq.y;
-  Rot32 r{1.f, 0.f, 1.f, 0.f};
-  if (g2 > 1e-17f) {
-    const float rg = rsqrtf(g2);
-    r.er = apq.x * rg;
-    r.ei = apq.y * rg;
-    const float zeta = 0.5f * (aqq - app) * rg;
-    const float h = 1.f + zeta * zeta;
-    const float t = copysignf(__fdividef(1.f, fabsf(zeta) + h * rsqrtf(h)), zeta);
-    r.c = rsqrtf(1.f + t * t);
-    r.s = t * r.c;
-    if (t * t > JAC32_ANGLE2 && g2 > JAC32_NOISE2) big = true;
-  }
-  return r;
-}
-// column k of the pair list of a round: index 0 stays, the others rotate (round < ne − 1)
-__device__ __forceinline__ int pair_pos(int k, int round, int ne) {
-  if (k == 0) return 0;
-  const int x = k - 1 + round;
-  return 1 + (x >= ne - 1 ? x - (ne - 1) : x);
+  const float g2 = fmaf(apq.x, apq.x, apq.y * apq.y), d = aqq - app, ad = fabsf(d) + 1e-9f;
+  const float rh = rsqrt_ftz(fmaf(ad, ad, 4.f * g2));
+  const float c2 = fmaf(0.5f * ad, rh, 0.5f);
+  const float rc = rsqrt_ftz(c2);
+  const float f = copysignf(rh * rc, d);
+  big |= (g2 > JAC32_NOISE2) & (g2 * f * f > JAC32_ANGLE2 * c2);
+  return Rot32{c2 * rc, make_float2(f * apq.x, f * apq.y)};
 }
 
-// Eigenvectors of the ne×ne (even; zero-padded) unit-norm Hermitian matrix `A` into V, the
-// eigenvalues on the diagonal of the buffer returned; A2 is scratch.  Thread items: the 2×2
-// blocks (pair, pair) of A, formed into the other buffer from their four old elements, and the
-// (pair, row) entries of V, updated in place; each thread computes the rotations it needs from
-// the old matrix, so a round is one barrier.
-__device__ inline float2* jacobi32(float2* A, float2* A2, float2* V, int ne, int ldf) {
+// The dynamic shared memory of k_rr; its matrices are addressed as offsets into it (an offset can be
+// swapped between buffers and the accesses stay shared-space ones).
+extern __shared__ __align__(16) unsigned char rr_smem_raw[];
+
+// Eigenvectors of the ne×ne (even; zero-padded) unit-norm Hermitian matrix at float2 offset oA into
+// oV, the eigenvalues on the diagonal of the matrix at the offset returned; the ne·ldf elements
+// after each are scratch (the other buffer).  Rows and columns are kept in the order of the
+// tournament, whose players all move to the next position after a round: position k always meets
+// ne − 1 − k, an element is read from one buffer and written at its next position in the other, so
+// every address is fixed, and a sweep of ne − 1 rounds ends in the order it began with.  A round is
+// two barriers: one thread per pair computes its rotation, then each thread takes the 2×2 blocks
+// (pair, pair) of A and the (pair, row) entries of V that are its items.  What counts is the number of
+// instructions in a warp's chain (≈4 cycles each): 10 K / 35 K / 284 K cycles
+// per matrix at n = 6 / 15 / 36, against 12 K / 53 K / 339 K with each thread working out its rotations and
+// addresses by itself in one-barrier rounds.
+template <int TL>
+__device__ inline int jacobi32(int oA, int oV, int ne, int ldf, float4* rots) {
   const int tid = threadIdx.x;
-  const int np = ne / 2, na = np * np, items = na + np * ne;
-  constexpr int SLOTS = 4;  // ne ≤ 36: na + np·ne ≤ 972
-  int ij[SLOTS];
+  const int np = ne / 2, na = np * np, v0 = (na + 31) & ~31;  // (whole warps take one kind of item)
+  constexpr int SLOTS = TL == 1 ? 1 : TL == 2 ? 3 : 4;        // ne ≤ 36: v0 + np·ne ≤ 1000
+  auto nx = [&](int k) { return k == 0 ? 0 : (k == ne - 1 ? 1 : k + 1); };
+  const uint32_t smem = (uint32_t)__cvta_generic_to_shared(rr_smem_raw), srot = (uint32_t)__cvta_generic_to_shared(rots);
+  const uint32_t sA = smem + 8 * oA, sV = smem + 8 * oV;
+  const bool pair = tid < np;
+  const int kp = pair ? tid : 0, ks = ne - 1 - kp;
+  const uint32_t r_ps = sA + 8 * (kp * ldf + ks), r_pp = sA + 8 * (kp * ldf + kp), r_ss = sA + 8 * (ks * ldf + ks);
+  // items: rotation addresses, the elements read (A: the block's corners; V: two) and written
+  uint32_t qa[SLOTS], qb[SLOTS], r_e[SLOTS][4], w_e[SLOTS][4];
+  int kind[SLOTS];
 #pragma unroll
   for (int q = 0; q < SLOTS; ++q) {
-    const int e = tid + q * EIG_NT;
-    const int w = e < na ? np : ne, b = e < na ? e : e - na;
-    ij[q] = e < items ? (b / w) | ((b % w) << 8) | (e < na ? 0 : 1 << 16) : -1;
+    const int e = tid + q * EIG_NT, ev = e - v0;
+    kind[q] = e < na ? 1 : (ev >= 0 && ev < np * ne ? 2 : 0);
+    const int I = e < na ? e / np : ev / ne, J = e < na ? e % np : ev % ne;
+    const int p = I, s = ne - 1 - I, u = J, v = ne - 1 - J;
+    qa[q] = srot + 16 * I;
+    qb[q] = srot + 16 * J;
+    if (e < na) {
+      r_e[q][0] = sA + 8 * (p * ldf + u); r_e[q][1] = sA + 8 * (p * ldf + v);
+      r_e[q][2] = sA + 8 * (s * ldf + u); r_e[q][3] = sA + 8 * (s * ldf + v);
+      w_e[q][0] = sA + 8 * (nx(p) * ldf + nx(u)); w_e[q][1] = sA + 8 * (nx(p) * ldf + nx(v));
+      w_e[q][2] = sA + 8 * (nx(s) * ldf + nx(u)); w_e[q][3] = sA + 8 * (nx(s) * ldf + nx(v));
+    } else {
+      r_e[q][0] = sV + 8 * (J * ldf + p); r_e[q][1] = sV + 8 * (J * ldf + s);
+      w_e[q][0] = sV + 8 * (J * ldf + nx(p)); w_e[q][1] = sV + 8 * (J * ldf + nx(s));
+      r_e[q][2] = r_e[q][3] = w_e[q][2] = w_e[q][3] = 0;
+    }
   }
-  float2* cur = A;
-  float2* nxt = A2;
+  uint32_t from = 0, to = 8 * ne * ldf;  // offsets of the buffer read and the one written
   for (int sweep = 0; sweep < 9; ++sweep) {
     bool big = false;
+#pragma unroll 1
     for (int round = 0; round < ne - 1; ++round) {
+      if (pair) {
+        const float2 aps = lds2(r_ps + from);
+        const float app = lds1(r_pp + from), ass = lds1(r_ss + from);
+        const Rot32 r = rot32(aps, app, ass, big);
+        sts4(srot + 16 * kp, make_float4(r.c, r.w.x, r.w.y, 0.f));
+      }
+      __syncthreads();
 #pragma unroll
       for (int q = 0; q < SLOTS; ++q) {
-        if (ij[q] < 0) break;
-        const int I = ij[q] & 255, J = (ij[q] >> 8) & 255;
-        const int p = pair_pos(I, round, ne), s = pair_pos(ne - 1 - I, round, ne);
-        const Rot32 a = rot32(cur[p * ldf + s], cur[p * ldf + p].x, cur[s * ldf + s].x, big);
-        const float2 ea = make_float2(a.er, a.ei), eac = make_float2(a.er, -a.ei);
-        if (ij[q] >> 16) {
-          const float2 vp = V[J * ldf + p], vs = cmulf(V[J * ldf + s], eac);
-          V[J * ldf + p] = make_float2(a.c * vp.x - a.s * vs.x, a.c * vp.y - a.s * vs.y);
-          V[J * ldf + s] = make_float2(a.s * vp.x + a.c * vs.x, a.s * vp.y + a.c * vs.y);
+        if (kind[q] == 0) continue;
+        const float4 a = lds4(qa[q]);
+        const float2 e0 = lds2(r_e[q][0] + from), e1 = lds2(r_e[q][1] + from);
+        const float2 aw = make_float2(a.y, a.z), ac = make_float2(a.y, -a.z);  // w, w̄
+        const float2 awn = make_float2(-a.y, -a.z), acn = make_float2(-a.y, a.z);
+        if (kind[q] == 2) {
+          sts2(w_e[q][0] + to, rotf(a.x, e0, acn, e1));
+          sts2(w_e[q][1] + to, rotf(a.x, e1, aw, e0));
         } else {
-          const int u = pair_pos(J, round, ne), v = pair_pos(ne - 1 - J, round, ne);
-          const Rot32 b = rot32(cur[u * ldf + v], cur[u * ldf + u].x, cur[v * ldf + v].x, big);
-          const float2 ebc = make_float2(b.er, -b.ei);
-          const float2 pu = cur[p * ldf + u], pv = cmulf(cur[p * ldf + v], ebc);
-          const float2 su = cmulf(cur[s * ldf + u], ea), sv = cmulf(cmulf(cur[s * ldf + v], ebc), ea);
-          // columns, then rows
-          const float2 p1 = make_float2(b.c * pu.x - b.s * pv.x, b.c * pu.y - b.s * pv.y);
-          const float2 p2 = make_float2(b.s * pu.x + b.c * pv.x, b.s * pu.y + b.c * pv.y);
-          const float2 s1 = make_float2(b.c * su.x - b.s * sv.x, b.c * su.y - b.s * sv.y);
-          const float2 s2 = make_float2(b.s * su.x + b.c * sv.x, b.s * su.y + b.c * sv.y);
-          const bool diag = I == J;
-          const float2 z = make_float2(0.f, 0.f);
-          nxt[p * ldf + u] = make_float2(a.c * p1.x - a.s * s1.x, diag ? 0.f : a.c * p1.y - a.s * s1.y);
-          nxt[p * ldf + v] = diag ? z : make_float2(a.c * p2.x - a.s * s2.x, a.c * p2.y - a.s * s2.y);
-          nxt[s * ldf + u] = diag ? z : make_float2(a.s * p1.x + a.c * s1.x, a.s * p1.y + a.c * s1.y);
-          nxt[s * ldf + v] = make_float2(a.s * p2.x + a.c * s2.x, diag ? 0.f : a.s * p2.y + a.c * s2.y);
+          const float4 b = lds4(qb[q]);
+          const float2 e2 = lds2(r_e[q][2] + from), e3 = lds2(r_e[q][3] + from);
+          const float2 bw = make_float2(b.y, b.z), bcn = make_float2(-b.y, b.z);
+          // columns, then rows (the annihilated pair is left at its rounding, below the noise that
+          // ends the sweeps)
+          const float2 p1 = rotf(b.x, e0, bcn, e1), p2 = rotf(b.x, e1, bw, e0);
+          const float2 s1 = rotf(b.x, e2, bcn, e3), s2 = rotf(b.x, e3, bw, e2);
+          sts2(w_e[q][0] + to, rotf(a.x, p1, awn, s1));
+          sts2(w_e[q][1] + to, rotf(a.x, p2, awn, s2));
+          sts2(w_e[q][2] + to, rotf(a.x, s1, ac, p1));
+          sts2(w_e[q][3] + to, rotf(a.x, s2, ac, p2));
         }
       }
       __syncthreads();
-      float2* t = cur; cur = nxt; nxt = t;
+      const uint32_t t = from; from = to; to = t;
     }
     if (!__syncthreads_or(big)) break;
   }
-  return cur;
+  return (int)(from / 8);
 }
 
 // Eigen-decomposition of the n×n Hermitian T (leading dimension ld, kept): the columns of the
-// matrix returned (X or Y) are the eigenvectors in ascending order up to rounding, lam their
-// eigenvalues.  W holds ld·(n + 1) double2 and is scratch, as is Y (the same size).  Returns nullptr where
+// matrix whose offset is returned (oX or oY) are the eigenvectors in ascending order up to rounding,
+// lam their eigenvalues.  Offsets count double2 in rr_smem_raw; W and Y hold ld·(n + 1) of them and
+// are scratch.  Returns −1 where
 // the refinement does not apply (non-finite or zero T; a pair with one of the lowest M columns too
 // close to be separated).  TL: 16×16 tiles per dimension covering n.
 template <int TL>
-__device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y, double2* W, int n, int M,
-                                        int ld, double* lam, double* red, int* order, double tol_e) {
+__device__ inline int eigh_refined(int oT, int oX, int oY, int oW, int n, int M, int ld, double* lam,
+                                   float* red, float4* rots, int* order, double tol_e) {
+  double2* const sm = reinterpret_cast<double2*>(rr_smem_raw);
+  const double2* const T = sm + oT;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int ne = n + (n & 1), ldf = ne | 1;
   // unit-norm FP32 copy, padded to an even size
@@ -263,17 +321,18 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
       const int i = ty + 16 * a, j = tx + 16 * b;
       if (i < n && j < n) { const double2 v = T[i * ld + j]; tot += v.x * v.x + v.y * v.y; }
     }
-  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-  if ((tid & 31) == 0) red[tid >> 5] = tot;
+  float totf = (float)tot;
+  for (int o = 16; o > 0; o >>= 1) totf += __shfl_xor_sync(0xffffffffu, totf, o);
+  if ((tid & 31) == 0) red[tid >> 5] = totf;
   __syncthreads();
-  tot = 0;
+  totf = 0;
 #pragma unroll
-  for (int w = 0; w < EIG_NT / 32; ++w) tot += red[w];
-  if (!(tot > 0) || !isfinite(tot)) return nullptr;
-  const double scale = rsqrt(tot);
-  float2* A = reinterpret_cast<float2*>(W);
-  float2* A2 = A + ne * ldf;
-  float2* V = reinterpret_cast<float2*>(Y);
+  for (int w = 0; w < EIG_NT / 32; ++w) totf += red[w];
+  if (!(totf > 1e-30f && totf < 1e30f)) return -1;
+  const double scale = rsqrtf(totf);
+  float2* const smf = reinterpret_cast<float2*>(rr_smem_raw);
+  float2* A = smf + 2 * oW;
+  float2* V = smf + 2 * oY;
   for (int i = ty; i < ne; i += 16)
     for (int j = tx; j < ne; j += 16) {
       const bool in = i < n && j < n;
@@ -282,8 +341,10 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
       V[i * ldf + j] = make_float2(i == j ? 1.f : 0.f, 0.f);
     }
   __syncthreads();
-  const float2* D = jacobi32(A, A2, V, ne, ldf);
-  // ascending order of the FP32 eigenvalues (the padding column is never moved, index n)
+  const int at = jacobi32<TL>(2 * oW, 2 * oY, ne, ldf, rots);
+  const float2* D = A + at;
+  V += at;
+  // ascending order of the FP32 eigenvalues (the padding stays at index n)
   if (tid < n) {
     const float d = D[tid * ldf + tid].x;
     int rank = 0;
@@ -297,11 +358,13 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
   for (int i = ty; i < n; i += 16)
     for (int j = tx; j < n; j += 16) {
       const float2 v = V[i * ldf + order[j]];
-      X[i * ld + j] = make_double2((double)v.x, (double)v.y);
+      sm[oX + i * ld + j] = make_double2((double)v.x, (double)v.y);
     }
   __syncthreads();
-  double2* E = W;
+  double2* const E = sm + oW;
   for (int step = 0; step < 6; ++step) {
+    const double2* X = sm + oX;
+    double2* Y = sm + oY;
     // Y = T X and R = I − XᴴX (into E)
     double2 t1[TL][TL], t2[TL][TL];
 #pragma unroll
@@ -312,17 +375,15 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
     for (int k = 0; k < n; ++k) {
       double2 xj[TL];
 #pragma unroll
-      for (int b = 0; b < TL; ++b) xj[b] = tx + 16 * b < n ? X[k * ld + tx + 16 * b] : make_double2(0, 0);
+      for (int b = 0; b < TL; ++b) xj[b] = X[k * ld + min(tx + 16 * b, n - 1)];
 #pragma unroll
       for (int a = 0; a < TL; ++a) {
-        const int i = ty + 16 * a;
-        if (i >= n) continue;
+        const int i = min(ty + 16 * a, n - 1);  // (threads outside the matrix repeat an edge)
         const double2 tik = T[i * ld + k], xi = X[k * ld + i];
 #pragma unroll
         for (int b = 0; b < TL; ++b) {
           t1[a][b] = cmac(t1[a][b], tik, xj[b]);
-          t2[a][b].x += xi.x * xj[b].x + xi.y * xj[b].y;  // conj(X_ki)·X_kj
-          t2[a][b].y += xi.x * xj[b].y - xi.y * xj[b].x;
+          t2[a][b] = cmacc(t2[a][b], xi, xj[b]);
         }
       }
     }
@@ -346,16 +407,14 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
     for (int k = 0; k < n; ++k) {
       double2 yj[TL];
 #pragma unroll
-      for (int b = 0; b < TL; ++b) yj[b] = tx + 16 * b < n ? Y[k * ld + tx + 16 * b] : make_double2(0, 0);
+      for (int b = 0; b < TL; ++b) yj[b] = Y[k * ld + min(tx + 16 * b, n - 1)];
 #pragma unroll
       for (int a = 0; a < TL; ++a) {
-        const int i = ty + 16 * a;
-        if (i >= n) continue;
+        const int i = min(ty + 16 * a, n - 1);  // (threads outside the matrix repeat an edge)
         const double2 xi = X[k * ld + i];
 #pragma unroll
         for (int b = 0; b < TL; ++b) {
-          t1[a][b].x += xi.x * yj[b].x + xi.y * yj[b].y;
-          t1[a][b].y += xi.x * yj[b].y - xi.y * yj[b].x;
+          t1[a][b] = cmacc(t1[a][b], xi, yj[b]);
         }
       }
     }
@@ -364,7 +423,7 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
 #pragma unroll
       for (int b = 0; b < TL; ++b) {
         const int i = ty + 16 * a, j = tx + 16 * b;
-        if (i == j && i < n) lam[i] = t1[a][b].x / (1.0 - t2[a][b].x);
+        if (i == j && i < n) lam[i] = t1[a][b].x * (1.0 + t2[a][b].x);  // 1/(1 − R_jj) to second order
       }
     __syncthreads();
     bool more = false, bad = false;
@@ -377,7 +436,8 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
         const double2 s = t1[a][b], r = t2[a][b];
         double2 e = make_double2(0.5 * r.x, 0.5 * r.y);
         if (i != j) {
-          const double lj = lam[j], inv = 1.0 / (lj - lam[i]);
+          const double lj = lam[j];
+          const double inv = (double)__frcp_rn((float)(lj - lam[i]));  // (a relative error of 1e-7: 1e-15 in a last step)
           const double2 f = make_double2((s.x + lj * r.x) * inv, (s.y + lj * r.y) * inv);
           const double f1 = fabs(f.x) + fabs(f.y);
           if (f1 <= E_MAX) e = f;             // (false for a NaN or infinite quotient)
@@ -390,7 +450,7 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
         if (e1 > tol_e) more = true;
         E[i * ld + j] = e;
       }
-    if (__syncthreads_or(bad)) return nullptr;
+    if (__syncthreads_or(bad)) return -1;
     // X ← X + X E, into Y
 #pragma unroll
     for (int a = 0; a < TL; ++a)
@@ -403,11 +463,10 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
     for (int k = 0; k < n; ++k) {
       double2 ej[TL];
 #pragma unroll
-      for (int b = 0; b < TL; ++b) ej[b] = tx + 16 * b < n ? E[k * ld + tx + 16 * b] : make_double2(0, 0);
+      for (int b = 0; b < TL; ++b) ej[b] = E[k * ld + min(tx + 16 * b, n - 1)];
 #pragma unroll
       for (int a = 0; a < TL; ++a) {
-        const int i = ty + 16 * a;
-        if (i >= n) continue;
+        const int i = min(ty + 16 * a, n - 1);  // (threads outside the matrix repeat an edge)
         const double2 xi = X[i * ld + k];
 #pragma unroll
         for (int b = 0; b < TL; ++b) t1[a][b] = cmac(t1[a][b], xi, ej[b]);
@@ -421,23 +480,10 @@ __device__ inline double2* eigh_refined(const double2* T, double2* X, double2* Y
         if (i < n && j < n) Y[i * ld + j] = t1[a][b];
       }
     more = __syncthreads_or(more);
-    double2* t = X; X = Y; Y = t;
-    if (!more) return X;
+    const int o = oX; oX = oY; oY = o;
+    if (!more) return oX;
   }
-  return nullptr;
-}
-
-// Indices of the eigenvalues (diagonal of A) in ascending order → order[0..n).
-__device__ inline void sort_diag(const double2* A, int n, int ld, int* order) {
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < n; ++i) order[i] = i;
-    for (int i = 1; i < n; ++i) {
-      int v = order[i], j = i - 1;
-      while (j >= 0 && A[order[j] * ld + order[j]].x > A[v * ld + v].x) { order[j + 1] = order[j]; --j; }
-      order[j + 1] = v;
-    }
-  }
-  __syncthreads();
+  return -1;
 }
 
 }  // namespace omb
