@@ -383,10 +383,7 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {  // conj(a)·b
-                acc[i][j].x += a[i].x * b[j].x + a[i].y * b[j].y;
-                acc[i][j].y += a[i].x * b[j].y - a[i].y * b[j].x;
-              }
+              for (int j = 0; j < 4; ++j) acc[i][j] = cmacc(acc[i][j], a[i], b[j]);  // conj(a)·b
           }
         }
       }

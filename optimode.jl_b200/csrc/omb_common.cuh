@@ -52,8 +52,9 @@ __device__ __forceinline__ float2 cmac(float2 acc, float2 a, float2 b) {
   acc = __ffma2_rn(make_float2(a.x, a.x), b, acc);
   return __ffma2_rn(make_float2(a.y, a.y), make_float2(-b.y, b.x), acc);
 }
+// FP64: four FMAs (summing the product first would take six operations)
 __device__ __forceinline__ double2 cmac(double2 acc, double2 a, double2 b) {
-  return make_double2(acc.x + (a.x * b.x - a.y * b.y), acc.y + (a.x * b.y + a.y * b.x));
+  return make_double2(fma(-a.y, b.y, fma(a.x, b.x, acc.x)), fma(a.y, b.x, fma(a.x, b.y, acc.y)));
 }
 // a * conj(b)
 template <typename C> __host__ __device__ __forceinline__ C cmulc(C a, C b) {
