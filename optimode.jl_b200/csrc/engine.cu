@@ -292,7 +292,7 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
   OMB_CU(gram_acc_.zero());
   OMB_CU(res_acc_.zero());
   // Lanes of tracks (split by Σ M², the Gram cost) run their iterations on separate streams,
-  // so one lane's latency-bound kernels (k_rr, k_control, k_newton, the prefix) overlap the
+  // so one lane's latency-bound kernels (k_rr, k_newton) overlap the
   // other lanes' streaming kernels.
   const int nl = std::max(1, std::min(LANES, nt_));
   int lane_lo[LANES], lane_hi[LANES];
@@ -365,26 +365,22 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
           return ok("HMkH pass", op(OP_HMKH, d_uH[par].p + off, cnt, g, 1));
         }))
       return e;
-    k_newton<<<(n + 127) / 128, 128, 0, s>>>(d_state_ptrs_.p + a, d_hmkh_ptrs_.p + a, d_hmkh_nb_.p + a, n, prm);
+    k_newton<<<1, NEWTON_NT, 0, s>>>(d_state_ptrs_.p + a, d_hmkh_ptrs_.p + a, d_hmkh_nb_.p + a, d_n2_.p + a, n, rg,
+                                     UpdCfg<T>::R, preg, preu, wpreg, wpreu, prm);
     if (!ok("k_newton", cudaGetLastError())) return e;
     if (!for_groups([&](const Group& g, int off, int cnt) {
           return ok("operator pass", op(OP_M, d_uA[par].p + off, cnt, g, 3 * g.Mmax));
         }))
       return e;
-    k_live_prefix<<<1, 1024, 0, s>>>(d_state_ptrs_.p + a, d_n2_.p + a, n, rg, UpdCfg<T>::R, preg, preu, wpreg,
-                                     wpreu);
-    if (!ok("k_live_prefix", cudaGetLastError())) return e;
     k_gram<T><<<grid_g, GramCfg<T>::NT, sm_gram, s>>>(d_descs.p + a, preg, wpreg, n, par, nmax, rg, gstages,
                                                        d_err_.p, ctx_->wait_ns);
     if (!ok("k_gram", cudaGetLastError())) return e;
     k_rr<<<n, RR_NT, sm_rr, s>>>(d_state_ptrs_.p + a, d_gram_ptrs_.p + a, d_coef_ptrs_.p + a, d_coef32_ptrs_.p + a, n,
                                  nmax, prm);
     if (!ok("k_rr", cudaGetLastError())) return e;
-    update_kernel<<<grid_u, UpdCfg<T>::NT, sm_upd, s>>>(d_descs.p + a, preu, wpreu, n, par, prm.prec_diag,
+    update_kernel<<<grid_u, UpdCfg<T>::NT, sm_upd, s>>>(d_descs.p + a, preu, wpreu, n, par, prm, d_ticket_.p + L,
                                                         d_err_.p, ctx_->wait_ns);
-    if (!ok("k_update", cudaGetLastError())) return e;
-    k_control<<<(n + 3) / 4, 128, 0, s>>>(d_state_ptrs_.p + a, d_res_ptrs_.p + a, n, prm);
-    ok("k_control", cudaGetLastError());
+    ok("k_update", cudaGetLastError());
     return e;
   };
 
@@ -497,10 +493,12 @@ int Engine::run() {
   OMB_CU(coef32_.zero());
   OMB_CU(d_err_.alloc(1, st));
   OMB_CU(d_err_.zero());
+  OMB_CU(d_ticket_.alloc(LANES, st));
+  OMB_CU(d_ticket_.zero());
   std::vector<TrackState*> sp(nt_);
   std::vector<double2*> gp(nt_), cp(nt_);
   std::vector<float2*> cp32(nt_);
-  std::vector<double*> rp(nt_), hp(nt_);
+  std::vector<double*> hp(nt_);
   std::vector<int> hnb(nt_);
   std::vector<long long> n2s(nt_);
   for (int gi = 0; gi < nt_; ++gi) {  // position gi holds track order_[gi]
@@ -510,7 +508,6 @@ int Engine::run() {
     gp[gi] = gram_acc_.p + (size_t)t * 2 * NMAX * NMAX;
     cp[gi] = coef_.p + (size_t)t * 2 * NMAX * MMAX;
     cp32[gi] = coef32_.p + (size_t)t * 2 * NMAX * MMAX;
-    rp[gi] = res_acc_.p + (size_t)t * MMAX;
     hp[gi] = hmkh_part_.p + (size_t)t * 2 * 512;
     hnb[gi] = row_blocks(P.Nx, P.Ny) * P.Nz;
     n2s[gi] = 2 * (long long)P.N();
@@ -522,13 +519,11 @@ int Engine::run() {
   OMB_CU(d_n2_.alloc(nt_, st));
   OMB_CU(cudaMemcpyAsync(d_coef32_ptrs_.p, cp32.data(), nt_ * sizeof(void*), cudaMemcpyHostToDevice, st));
   OMB_CU(cudaMemcpyAsync(d_n2_.p, n2s.data(), nt_ * sizeof(long long), cudaMemcpyHostToDevice, st));
-  OMB_CU(d_res_ptrs_.alloc(nt_, st));
   OMB_CU(d_hmkh_ptrs_.alloc(nt_, st));
   OMB_CU(d_hmkh_nb_.alloc(nt_, st));
   OMB_CU(cudaMemcpyAsync(d_state_ptrs_.p, sp.data(), nt_ * sizeof(void*), cudaMemcpyHostToDevice, st));
   OMB_CU(cudaMemcpyAsync(d_gram_ptrs_.p, gp.data(), nt_ * sizeof(void*), cudaMemcpyHostToDevice, st));
   OMB_CU(cudaMemcpyAsync(d_coef_ptrs_.p, cp.data(), nt_ * sizeof(void*), cudaMemcpyHostToDevice, st));
-  OMB_CU(cudaMemcpyAsync(d_res_ptrs_.p, rp.data(), nt_ * sizeof(void*), cudaMemcpyHostToDevice, st));
   OMB_CU(cudaMemcpyAsync(d_hmkh_ptrs_.p, hp.data(), nt_ * sizeof(void*), cudaMemcpyHostToDevice, st));
   OMB_CU(cudaMemcpyAsync(d_hmkh_nb_.p, hnb.data(), nt_ * sizeof(int), cudaMemcpyHostToDevice, st));
   OMB_CU(cudaStreamSynchronize(st));

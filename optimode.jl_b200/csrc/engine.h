@@ -103,12 +103,13 @@ class Engine {
   DevBuf<TrackState*> d_state_ptrs_;
   DevBuf<double2*> d_gram_ptrs_, d_coef_ptrs_;
   DevBuf<float2*> d_coef32_ptrs_;
-  DevBuf<double*> d_res_ptrs_, d_hmkh_ptrs_;
+  DevBuf<double*> d_hmkh_ptrs_;
   DevBuf<int> d_hmkh_nb_;
   DevBuf<long long> d_n2_;
   DevBuf<int> d_pre_;   // live-tile prefixes: Gram tiles [0, nt], update tiles [nt+1, 2nt+1]
   DevBuf<long long> d_wpre_;  // the same prefixes weighted by each tile's cost
   DevBuf<int> d_err_;   // first pipeline error of the streaming kernels (0: none)
+  DevBuf<unsigned> d_ticket_;  // k_update's arrival counter of each lane
 
   // block buffers of the current precision (Y/AY per parity, scratch)
   DevBuf<float2> y32_, s32_;

@@ -33,6 +33,7 @@ constexpr int MMAX = 12;         // block columns per track
 constexpr int NMAX = 3 * MMAX;   // Rayleigh–Ritz basis size
 constexpr int LANES = 2;         // track lanes (streams) of an engine's iteration graph
 constexpr int RR_NT = EIG_NT;
+constexpr int NEWTON_NT = 256;
 
 enum TrackStatus : int {
   TS_RUNNING = 0, TS_CONVERGED = 1, TS_MAXITER = 2, TS_ORTHO = 3, TS_NAN = 4, TS_PHASE_DONE = 5,
@@ -98,11 +99,11 @@ __device__ __forceinline__ int z_phys(const TrackState& s, int M, int l) {
 // Both stream the row tiles of the live tracks through shared memory with bulk copies
 // (one producer warp, a ring of `stages` buffers guarded by full/empty mbarriers) while
 // the consumer warps compute.  The rows of all live tracks form one sequence of tiles
-// (k_live_prefix counts them after the Newton step of the iteration); CTA b of a 1D grid
+// (k_newton counts them after the Newton step of the iteration); CTA b of a 1D grid
 // of X takes the tiles that start in [b·W/X, (b+1)·W/X) of the tiles' summed cost W (a
 // tile of a wide track costs several times one of a narrow track), so the work stays
 // spread evenly over every SM however few tracks are left.  Per-track sums leave each CTA through FP64 atomics into the
-// track's accumulators, which k_rr (Gram) and k_control (‖R‖²) read and clear.
+// track's accumulators, which k_rr (Gram) and control_track (‖R‖²) read and clear.
 
 // Tile sequence of one CTA: tiles of R rows of the live tracks, in track order.
 struct TileWalk {
@@ -157,11 +158,6 @@ struct TileWalk {
   __device__ __forceinline__ bool last_of_track() const { return i + 1 >= end || pre[t + 1] <= i + 1; }
 };
 
-// Live-tile prefixes for the Gram (rows per tile rg) and update (ru) kernels, and the
-// prefixes of their cost-weighted tile counts (wpre_g, wpre_u).
-__global__ void k_live_prefix(TrackState* const* __restrict__ states, const long long* __restrict__ n2,
-                              int ntracks, int rg, int ru, int* __restrict__ pre_g, int* __restrict__ pre_u,
-                              long long* __restrict__ wpre_g, long long* __restrict__ wpre_u);
 // Relative cost of one tile of a track with n block columns of which M are X: the Gram's 4×4
 // items (each 16 complex products per row) plus its loads plus a fixed GRAM_TILE_FIXED, and
 // GRAM_TRACK_COST once per track for the flush of its sums (each CTA that takes part in a
@@ -445,6 +441,75 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
   }
 }
 
+// ---- Control ---------------------------------------------------------------------
+__device__ __forceinline__ void finish(TrackState& s, int status) {
+  s.status = status;
+  s.done = 1;
+  s.op_ncol = 0; s.pw_ncol = 0; s.hmkh_ncol = 0;
+}
+
+// The decisions after an update, for one track (one thread): residual norms from the sums of
+// k_update (cleared for the next iteration), locking, the phase's exits, and whether a Newton step
+// is due.
+__device__ inline void control_track(TrackState& s, double* ra, const IterParams& prm) {
+  if (s.done) return;
+  const int M = s.M;
+  double rs[MMAX];
+  for (int m = 0; m < M; ++m) { rs[m] = __ldcg(ra + m); ra[m] = 0.0; }
+  bool bad = false;
+  for (int m = 0; m < M; ++m) {
+    s.resid[m] = sqrt(rs[m]);
+    if (!isfinite(s.resid[m]) || !isfinite(s.lam[m])) bad = true;
+  }
+  s.nP = s.nP_next;
+  s.iter++; s.iter_phase++; s.since_newton++;
+  if (bad || !isfinite(s.k)) { finish(s, TS_NAN); return; }
+  const int need = s.need;
+  double maxres = 0;
+  for (int i = 0; i < need; ++i) maxres = fmax(maxres, s.resid[i]);
+  if (maxres < 0.9 * s.resid_best) { s.resid_best = maxres; s.stall = 0; } else { s.stall++; }
+  while (s.nlocked < need && s.resid[s.nlocked] < prm.lock_tol) s.nlocked++;
+  const bool last = prm.last_phase != 0;
+  s.hmkh_ncol = 0;
+  if (s.mode == MODE_OMEGA2) {
+    if (maxres < prm.tau_phase) { finish(s, last ? TS_CONVERGED : TS_PHASE_DONE); return; }
+    if (!last && s.stall >= 8) { finish(s, TS_PHASE_DONE); return; }
+  } else if (s.mode == MODE_NEWTON_INNER) {
+    const double dw2 = s.lam[s.band] - s.omega2;
+    if (last) {
+      // final steps from converged eigenpairs; earlier ones while the k mismatch dominates
+      // the eigen-residual, plus at most one early step per phase near the tolerance.  The
+      // track returns band `band` only, and that Ritz pair's own residual bounds its error,
+      // so the polish watches it alone; the lower bands (resolved to the FP32 floor before
+      // the hand-over, which keeps the Ritz ordering) keep iterating beside it.
+      const double rb = s.resid[s.band];
+      if (rb < prm.tol) s.hmkh_ncol = 1;
+      else if (s.since_newton >= 2 && rb < 0.1 * fabs(dw2)) s.hmkh_ncol = 1;
+      else if (s.since_newton >= 2 && s.newton_phase == 0 && rb < 100 * prm.tol) s.hmkh_ncol = 1;
+    } else {
+      if (s.newton_steps > 0 && maxres < prm.tau_phase && fabs(s.dk_last) < prm.dk_phase) {
+        finish(s, TS_PHASE_DONE); return;
+      }
+      // stalled at the FP32 floor: the FP64 phase takes over, with or without a Newton step
+      // here (a warm start can give a k so close that λ_b − ω² never dominates the
+      // residual); plateaus far above the floor keep iterating in FP32
+      const bool at_floor = maxres < 4.0 * prm.tau_phase;
+      if (at_floor && s.stall >= 8) { finish(s, TS_PHASE_DONE); return; }
+      if (s.newton_steps > 0 && s.stall >= 8) { finish(s, TS_PHASE_DONE); return; }
+      if (s.since_newton >= 2 && (maxres < fmax(0.1 * fabs(dw2), prm.tau_phase) || (at_floor && s.stall >= 4)))
+        s.hmkh_ncol = 1;
+    }
+  } else {  // MODE_NEWTON_OUTER: the reference loop, a step after each converged eigensolve
+    if (maxres < prm.tol) s.hmkh_ncol = 1;
+  }
+  if (s.iter_phase >= prm.maxiter && s.hmkh_ncol == 0) { finish(s, last ? TS_MAXITER : TS_PHASE_DONE); return; }
+  s.nWa = M - s.nlocked;
+  s.op_col0 = M + s.nlocked;
+  s.op_ncol = s.nWa;
+  s.pw_col0 = s.nlocked;
+  s.pw_ncol = s.nWa;
+}
+
 // ---- Update -----------------------------------------------------------------------
 // X ← ZC, AX ← AZC, P ← ZCP, AP ← AZCP into the other parity, then R = AX − XΛ,
 // W = P̂_diag R (or R when the MPB preconditioner follows) and ‖R‖².  One consumer thread
@@ -553,7 +618,8 @@ __device__ __forceinline__ void update_tile(const TrackDesc<T>& d, const TrackSt
 template <typename T, int MB>
 __global__ void __launch_bounds__(UpdCfg<T>::NT, 1)
     k_update(const TrackDesc<T>* __restrict__ D, const int* __restrict__ pre, const long long* __restrict__ wpre,
-             int ntracks, int par, int prec_diag, int* __restrict__ err, uint64_t wait_ns) {
+             int ntracks, int par, IterParams prm, unsigned* __restrict__ ticket, int* __restrict__ err,
+             uint64_t wait_ns) {
   using C = cplx<T>;
   using Cfg = UpdCfg<T>;
   constexpr int R = Cfg::R, LG = Cfg::LG, S = Cfg::STAGES;
@@ -611,42 +677,57 @@ __global__ void __launch_bounds__(UpdCfg<T>::NT, 1)
       for (int k = 0; k < S; ++k)
         if (fills[k] > 0 && !mbar_wait(&full[k], (uint32_t)((fills[k] - 1) & 1), drain_limit(wait_ns)))
           pipe_fail(err, PIPE_DRAIN_TIMEOUT);
-    return;
-  }
-  // ---- consumers: thread r owns row row0 + r of each tile
-  int q = 0;
-  uint32_t ph = 0;
-  bool failed = false;
-  double racc[MB];
+  } else {
+    // ---- consumers: thread r owns row row0 + r of each tile
+    int q = 0;
+    uint32_t ph = 0;
+    bool failed = false;
+    double racc[MB];
 #pragma unroll
-  for (int m = 0; m < MB; ++m) racc[m] = 0;
-  for (; w.valid(); w.next()) {
-    const TrackDesc<T>& d = D[w.t];
-    const TrackState& s = *d.st;
-    if (s.done) continue;
-    const long long r0 = w.row0();
-    const int rows = (int)min((long long)R, d.n2 - r0);
-    switch (d.M) {
+    for (int m = 0; m < MB; ++m) racc[m] = 0;
+    for (; w.valid(); w.next()) {
+      const TrackDesc<T>& d = D[w.t];
+      const TrackState& s = *d.st;
+      if (s.done) continue;
+      const long long r0 = w.row0();
+      const int rows = (int)min((long long)R, d.n2 - r0);
+      switch (d.M) {
 #define OMB_UPD_CASE(MM)                                                                                \
-  case MM:                                                                                              \
-    if constexpr (MM <= MB)                                                                             \
-      update_tile<T, (MM <= MB ? MM : 1), MB>(d, s, r0, rows, par, prec_diag, stage0, full, empty, q, ph, \
-                                              failed, racc, err, wait_ns);                              \
-    break;
-      OMB_UPD_CASE(1) OMB_UPD_CASE(2) OMB_UPD_CASE(3) OMB_UPD_CASE(4) OMB_UPD_CASE(5) OMB_UPD_CASE(6)
-      OMB_UPD_CASE(7) OMB_UPD_CASE(8) OMB_UPD_CASE(9) OMB_UPD_CASE(10) OMB_UPD_CASE(11) OMB_UPD_CASE(12)
+    case MM:                                                                                              \
+      if constexpr (MM <= MB)                                                                             \
+        update_tile<T, (MM <= MB ? MM : 1), MB>(d, s, r0, rows, par, prm.prec_diag, stage0, full, empty, q, ph, \
+                                                failed, racc, err, wait_ns);                              \
+      break;
+        OMB_UPD_CASE(1) OMB_UPD_CASE(2) OMB_UPD_CASE(3) OMB_UPD_CASE(4) OMB_UPD_CASE(5) OMB_UPD_CASE(6)
+        OMB_UPD_CASE(7) OMB_UPD_CASE(8) OMB_UPD_CASE(9) OMB_UPD_CASE(10) OMB_UPD_CASE(11) OMB_UPD_CASE(12)
 #undef OMB_UPD_CASE
-      default: break;
-    }
-    if (w.last_of_track()) {
+        default: break;
+      }
+      if (w.last_of_track()) {
 #pragma unroll
-      for (int m = 0; m < MB; ++m) {
-        double v = racc[m];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0 && m < d.M && !failed) atomicAdd(d.res_acc + m, v);
-        racc[m] = 0;
+        for (int m = 0; m < MB; ++m) {
+          double v = racc[m];
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == 0 && m < d.M && !failed) atomicAdd(d.res_acc + m, v);
+          racc[m] = 0;
+        }
       }
     }
+  }
+  // The last CTA to get here takes the iteration's decisions, a thread per track (as a kernel of its own
+  // they took 6–7 µs of every iteration): every other CTA has made its sums visible (fence, then
+  // ticket) and reads no track state any more.
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    if (threadIdx.x == 0) *ticket = 0;
+    for (int t = threadIdx.x; t < ntracks; t += Cfg::NT) control_track(*D[t].st, D[t].res_acc, prm);
   }
 }
 
@@ -666,12 +747,13 @@ __host__ __device__ constexpr size_t rr_mat(int nmax) { return (size_t)((nmax + 
 __host__ __device__ constexpr size_t rr_smem(int nmax) { return 5 * rr_mat(nmax) * sizeof(double2); }
 
 // ---------------------------------------------------------------------------------
-// Control (after the update; one warp per track) and Newton (after the HMkH pass; one
-// thread per track).
-__global__ void k_control(TrackState* const* __restrict__ states, double* const* __restrict__ res_accs,
-                          int ntracks, IterParams prm);
-__global__ void k_newton(TrackState* const* __restrict__ states, double* const* __restrict__ hmkh_parts,
-                         const int* __restrict__ hmkh_nb, int ntracks, IterParams prm);
+// Newton steps (after the HMkH pass) and the live-tile prefixes for the Gram (rows per tile rg) and
+// update (ru) kernels: tile counts (pre_*) and cost-weighted tile counts (wpre_*).  One CTA.
+__global__ void __launch_bounds__(NEWTON_NT)
+    k_newton(TrackState* const* __restrict__ states, double* const* __restrict__ hmkh_parts,
+             const int* __restrict__ hmkh_nb, const long long* __restrict__ n2, int ntracks, int rg, int ru,
+             int* __restrict__ pre_g, int* __restrict__ pre_u, long long* __restrict__ wpre_g,
+             long long* __restrict__ wpre_u, IterParams prm);
 
 // Random start block (uniform in [-1,1]² per entry from a counter-based hash).
 template <typename T>
