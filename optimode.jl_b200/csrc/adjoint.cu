@@ -18,7 +18,10 @@
 // Givens rotations are real, only the vectors are complex.  Every vector stays orthogonal to
 // h (the right-hand side is, and the preconditioned vector is projected), which deflates the
 // eigenvalue ω² of the operator.  All recurrence scalars live in device memory; one
-// iteration is a fixed launch sequence replayed from a CUDA graph.
+// iteration is a fixed launch sequence replayed from a CUDA graph: the three operator passes and three
+// vector kernels, whose last CTA sums the dot products and takes the scalar step.  Every band of the
+// pull-back is a row of each launch: a solve is bound by the latency of its launches (a vector of a
+// 256² cell is 2 MB, resident in L2), not by bytes, so the bands share it.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -38,6 +41,7 @@ struct MinresState {
   double dot_ey_r, dot_ey_i, dot_ez_r, dot_ez_i;
   double rtol;
   double phibar_mark;  // phibar at itn_mark (stagnation test)
+  int active;          // operator columns of the solve (0 once it is over)
   int itn, maxit, done, status;  // status: 0 running, 1 converged, 2 maxiter, 3 breakdown,
                                  // 4 maxiter with the residual below LOOSE_TOL
   int itn_mark;
@@ -62,75 +66,124 @@ constexpr double LOOSE_TOL = 1.4901161193847656e-08;
 constexpr double FLAT_TOL = 1e-6;
 constexpr int FLAT_WINDOWS = 4;
 
+// Sums of four doubles over the CTA, valid in thread 0 (every thread calls it).
+__device__ __forceinline__ void block_sum4(double (&v)[4]) {
+  __shared__ double sm[4][ADJ_NT / 32];
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sm[q][w] = v[q];
+  __syncthreads();
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      double s = 0;
+      for (int i = 0; i < ADJ_NT / 32; ++i) s += sm[q][i];
+      v[q] = s;
+    }
+  __syncthreads();
+}
+
 // block-reduce two complex partial sums (4 doubles) into part[blockIdx.x*4 + 0..3]
 __device__ __forceinline__ void block_reduce4(double a, double b, double c, double d, double* part) {
-  __shared__ double sm[4][ADJ_NT / 32];
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-    d += __shfl_xor_sync(0xffffffffu, d, o);
-  }
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) { sm[0][w] = a; sm[1][w] = b; sm[2][w] = c; sm[3][w] = d; }
+  double v[4] = {a, b, c, d};
+  block_sum4(v);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) part[4 * blockIdx.x + q] = v[q];
+}
+
+// Arrival of a CTA of row blockIdx.y of the grid: true in every thread of the last one, which resets
+// the counter.  What the others wrote before is then visible.
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int i = 0; i < ADJ_NT / 32; ++i) { s0 += sm[0][i]; s1 += sm[1][i]; s2 += sm[2][i]; s3 += sm[3][i]; }
-    part[4 * blockIdx.x + 0] = s0;
-    part[4 * blockIdx.x + 1] = s1;
-    part[4 * blockIdx.x + 2] = s2;
-    part[4 * blockIdx.x + 3] = s3;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0;
   }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
 }
 
-struct AdjVecs {
+// Grid-wide sums: block partials, then the last CTA adds them with all its threads in a fixed order.
+// True in thread 0 of that CTA, with the sums in v.  (One thread adding 296 partials in a kernel of its
+// own took ≈10 µs.)
+__device__ __forceinline__ bool grid_sum4(double (&v)[4], double* part, unsigned* ticket) {
+  block_reduce4(v[0], v[1], v[2], v[3], part);
+  if (!last_block(ticket)) return false;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = 0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += ADJ_NT)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] += __ldcg(part + 4 * i + q);
+  block_sum4(v);
+  return threadIdx.x == 0;
+}
+
+// One band's solve: all bands of a pull-back run together, a row of CTAs (blockIdx.y) each.
+struct AdjBand {
   double2 *x, *v, *w, *w2, *r1, *r2, *y, *Av;
+  double2* b;        // right-hand side
   const double2* e;  // unit eigenvector (deflation direction)
-  long long n2;
-  int Nx, Ny;
-  double inv_dx, inv_dy, k, eps_mean;
-  int Nz;            // z-periodic cells (1 for a 2D cell)
-  double inv_dz;
+  double* part;      // partial sums, 4 per CTA
+  unsigned* ticket;
+  MinresState* S;
+  double k;
+};
+struct AdjGeom {
+  int N, Nx, Ny, Nz;  // pixels (two coefficients each); Nz = 1 for a 2D cell
+  double inv_dx, inv_dy, inv_dz, eps_mean;
 };
 
-// Diagonal preconditioner ⟨ε⟩/|w|² at row `row` (w = k ẑ − G; g_z of the row's slab)
-__device__ __forceinline__ double prec_scale(long long row, const AdjVecs& V) {
-  const long long p = row >> 1;
-  const int ix = (int)(p % V.Nx);
-  const long long rest = p / V.Nx;
-  const int iy = (int)(rest % V.Ny), iz = (int)(rest / V.Ny);
-  const double gx = freq_index(ix, V.Nx) * V.inv_dx, gy = freq_index(iy, V.Ny) * V.inv_dy;
-  const double wz = V.k - freq_index(iz, V.Nz) * V.inv_dz;
-  return V.eps_mean / (gx * gx + gy * gy + wz * wz);
+// Diagonal preconditioner ⟨ε⟩/|w|² at pixel p (w = k ẑ − G; g_z of the pixel's slab)
+__device__ __forceinline__ double prec_scale(unsigned p, const AdjGeom& G, double k) {
+  const unsigned rest = p / (unsigned)G.Nx, ix = p - rest * (unsigned)G.Nx;
+  const unsigned iz = rest / (unsigned)G.Ny, iy = rest - iz * (unsigned)G.Ny;
+  const double gx = freq_index((int)ix, G.Nx) * G.inv_dx, gy = freq_index((int)iy, G.Ny) * G.inv_dy;
+  const double wz = k - freq_index((int)iz, G.Nz) * G.inv_dz;
+  return G.eps_mean / (gx * gx + gy * gy + wz * wz);
 }
 
-// init: r1 = r2 = b, z = P b, partials ⟨e,z⟩, ⟨b,z⟩ (y holds z)
-__global__ void __launch_bounds__(ADJ_NT) k_minres_init(AdjVecs V, const double2* __restrict__ b, double* part) {
-  double er = 0, ei = 0, br = 0, bi = 0;
-  for (long long i = blockIdx.x * (long long)ADJ_NT + threadIdx.x; i < V.n2; i += (long long)gridDim.x * ADJ_NT) {
-    const double2 bb = b[i];
-    const double s = prec_scale(i, V);
-    const double2 z = make_double2(bb.x * s, bb.y * s);
-    V.r1[i] = bb; V.r2[i] = bb; V.y[i] = z;
-    V.x[i] = make_double2(0, 0); V.w[i] = make_double2(0, 0); V.w2[i] = make_double2(0, 0);
-    const double2 e = V.e[i];
-    er += e.x * z.x + e.y * z.y; ei += e.x * z.y - e.y * z.x;   // conj(e)·z
-    br += bb.x * z.x + bb.y * z.y; bi += bb.x * z.y - bb.y * z.x;
+__device__ __forceinline__ void dot_acc(double& re, double& im, double2 a, double2 b) {  // += conj(a)·b
+  re += a.x * b.x + a.y * b.y;
+  im += a.x * b.y - a.y * b.x;
+}
+// a − c·b for a complex c
+__device__ __forceinline__ double2 sub_mul(double2 a, double cr, double ci, double2 b) {
+  return make_double2(a.x - (cr * b.x - ci * b.y), a.y - (cr * b.y + ci * b.x));
+}
+
+// init: r1 = r2 = b, z = P b, partials ⟨e,z⟩, ⟨b,z⟩ (y holds z); then the scalars
+__global__ void __launch_bounds__(ADJ_NT) k_minres_init(const AdjBand* __restrict__ bands, AdjGeom G) {
+  const AdjBand V = bands[blockIdx.y];
+  double d[4] = {0, 0, 0, 0};
+  for (int p = blockIdx.x * ADJ_NT + threadIdx.x; p < G.N; p += gridDim.x * ADJ_NT) {
+    const double s = prec_scale(p, G, V.k);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const size_t i = 2 * (size_t)p + c;
+      const double2 bb = V.b[i], zero = make_double2(0, 0);
+      const double2 z = make_double2(bb.x * s, bb.y * s);
+      V.r1[i] = bb; V.r2[i] = bb; V.y[i] = z;
+      V.x[i] = zero; V.w[i] = zero; V.w2[i] = zero;
+      dot_acc(d[0], d[1], V.e[i], z);
+      dot_acc(d[2], d[3], bb, z);
+    }
   }
-  block_reduce4(er, ei, br, bi, part);
-}
-
-__global__ void k_minres_init_scalar(MinresState* S, const double* part, int nb) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double er = 0, ei = 0, br = 0;
-  for (int i = 0; i < nb; ++i) { er += part[4 * i]; ei += part[4 * i + 1]; br += part[4 * i + 2]; }
-  S->dot_ez_r = er; S->dot_ez_i = ei;
-  const double b2 = br;
-  S->itn = 0; S->done = 0; S->status = 0;
+  if (!grid_sum4(d, V.part, V.ticket)) return;
+  MinresState* S = V.S;
+  S->dot_ez_r = d[0]; S->dot_ez_i = d[1];
+  const double b2 = d[2];
+  S->itn = 0; S->done = 0; S->status = 0; S->active = 1;
   S->oldb = 0; S->dbar = 0; S->epsln = 0; S->oldeps = 0; S->cs = -1; S->sn = 0;
   if (!(b2 > 0) || !isfinite(b2)) {  // zero right-hand side: λ = 0
-    S->beta1 = S->beta = 0; S->phibar = 0; S->done = 1; S->status = 1;
+    S->beta1 = S->beta = 0; S->phibar = 0; S->done = 1; S->status = 1; S->active = 0;
     return;
   }
   S->beta1 = S->beta = sqrt(b2);
@@ -141,65 +194,39 @@ __global__ void k_minres_init_scalar(MinresState* S, const double* part, int nb)
 }
 
 // v = (z − ⟨e,z⟩e)/beta  (start of the first iteration)
-__global__ void __launch_bounds__(ADJ_NT) k_minres_first_v(AdjVecs V, const MinresState* S) {
+__global__ void __launch_bounds__(ADJ_NT) k_minres_first_v(const AdjBand* __restrict__ bands, AdjGeom G) {
+  const AdjBand V = bands[blockIdx.y];
+  const MinresState* S = V.S;
   if (S->done) return;
   const double inv = 1.0 / S->beta, er = S->dot_ez_r, ei = S->dot_ez_i;
-  for (long long i = blockIdx.x * (long long)ADJ_NT + threadIdx.x; i < V.n2; i += (long long)gridDim.x * ADJ_NT) {
-    const double2 z = V.y[i], e = V.e[i];
-    V.v[i] = make_double2((z.x - (er * e.x - ei * e.y)) * inv, (z.y - (er * e.y + ei * e.x)) * inv);
+  for (int i = blockIdx.x * ADJ_NT + threadIdx.x; i < 2 * G.N; i += gridDim.x * ADJ_NT) {
+    const double2 z = sub_mul(V.y[i], er, ei, V.e[i]);
+    V.v[i] = make_double2(z.x * inv, z.y * inv);
   }
 }
 
-// y = Av − shift·v − (beta/oldb)·r1 ; partials ⟨e,y⟩, ⟨v,y⟩
-__global__ void __launch_bounds__(ADJ_NT) k_minres_a(AdjVecs V, const MinresState* S, double* part) {
+// y = Av − shift·v − (beta/oldb)·r1 ; sums ⟨e,y⟩, ⟨v,y⟩ = alfa (real for a Hermitian operator, v ⟂ e)
+__global__ void __launch_bounds__(ADJ_NT) k_minres_a(const AdjBand* __restrict__ bands, AdjGeom G) {
+  const AdjBand V = bands[blockIdx.y];
+  MinresState* S = V.S;
   if (S->done) return;
   const double sh = S->shift;
   const double c1 = S->itn >= 1 ? S->beta / S->oldb : 0.0;
-  double er = 0, ei = 0, vr = 0, vi = 0;
-  for (long long i = blockIdx.x * (long long)ADJ_NT + threadIdx.x; i < V.n2; i += (long long)gridDim.x * ADJ_NT) {
+  double d[4] = {0, 0, 0, 0};
+  for (int i = blockIdx.x * ADJ_NT + threadIdx.x; i < 2 * G.N; i += gridDim.x * ADJ_NT) {
     const double2 av = V.Av[i], v = V.v[i], r1 = V.r1[i], e = V.e[i];
     const double2 y = make_double2(av.x - sh * v.x - c1 * r1.x, av.y - sh * v.y - c1 * r1.y);
     V.y[i] = y;
-    er += e.x * y.x + e.y * y.y; ei += e.x * y.y - e.y * y.x;
-    vr += v.x * y.x + v.y * y.y; vi += v.x * y.y - v.y * y.x;
+    dot_acc(d[0], d[1], e, y);
+    dot_acc(d[2], d[3], v, y);
   }
-  block_reduce4(er, ei, vr, vi, part);
-}
-
-__global__ void k_minres_a_scalar(MinresState* S, const double* part, int nb) {
-  if (threadIdx.x != 0 || blockIdx.x != 0 || S->done) return;
-  double er = 0, ei = 0, vr = 0;
-  for (int i = 0; i < nb; ++i) { er += part[4 * i]; ei += part[4 * i + 1]; vr += part[4 * i + 2]; }
-  S->dot_ey_r = er; S->dot_ey_i = ei;
-  S->alfa = vr;  // ⟨v, y⟩ is real for a Hermitian operator (v ⟂ e)
-}
-
-// y ← y − ⟨e,y⟩e − (alfa/beta) r2 ; r1 ← r2 ; r2 ← y ; z = P r2 (into y) ; partials ⟨e,z⟩, ⟨r2,z⟩
-__global__ void __launch_bounds__(ADJ_NT) k_minres_b(AdjVecs V, const MinresState* S, double* part) {
-  if (S->done) return;
-  const double c2 = S->alfa / S->beta, er0 = S->dot_ey_r, ei0 = S->dot_ey_i;
-  double er = 0, ei = 0, rr = 0, ri = 0;
-  for (long long i = blockIdx.x * (long long)ADJ_NT + threadIdx.x; i < V.n2; i += (long long)gridDim.x * ADJ_NT) {
-    const double2 y = V.y[i], e = V.e[i], r2 = V.r2[i];
-    const double2 yn = make_double2(y.x - (er0 * e.x - ei0 * e.y) - c2 * r2.x, y.y - (er0 * e.y + ei0 * e.x) - c2 * r2.y);
-    V.r1[i] = r2;
-    V.r2[i] = yn;
-    const double s = prec_scale(i, V);
-    const double2 z = make_double2(yn.x * s, yn.y * s);
-    V.y[i] = z;
-    er += e.x * z.x + e.y * z.y; ei += e.x * z.y - e.y * z.x;
-    rr += yn.x * z.x + yn.y * z.y; ri += yn.x * z.y - yn.y * z.x;
-  }
-  block_reduce4(er, ei, rr, ri, part);
+  if (!grid_sum4(d, V.part, V.ticket)) return;
+  S->dot_ey_r = d[0]; S->dot_ey_i = d[1];
+  S->alfa = d[2];
 }
 
 // Lanczos coefficient β_{k+1} and the Givens rotation of MINRES (all real)
-__global__ void k_minres_b_scalar(MinresState* S, const double* part, int nb) {
-  if (threadIdx.x != 0 || blockIdx.x != 0 || S->done) return;
-  double er = 0, ei = 0, rr = 0;
-  for (int i = 0; i < nb; ++i) { er += part[4 * i]; ei += part[4 * i + 1]; rr += part[4 * i + 2]; }
-  S->dot_ez_r = er; S->dot_ez_i = ei;
-  const double b2 = rr;  // ⟨r2, z − e⟨e,z⟩⟩ = ⟨r2, z⟩ since r2 ⟂ e
+__device__ __forceinline__ void minres_rotate(MinresState* S, double b2) {
   S->oldb = S->beta;
   S->beta = b2 > 0 ? sqrt(b2) : 0.0;
   S->oldeps = S->epsln;
@@ -216,7 +243,7 @@ __global__ void k_minres_b_scalar(MinresState* S, const double* part, int nb) {
   S->phi = S->cs * S->phibar;
   S->phibar = S->sn * S->phibar;
   S->itn++;
-  if (!isfinite(S->phibar) || !isfinite(S->phi)) { S->done = 1; S->status = 3; return; }
+  if (!isfinite(S->phibar) || !isfinite(S->phi)) { S->done = 1; S->status = 3; S->active = 0; return; }
   if (S->phibar <= S->rtol * S->beta1) { S->done = 2; S->status = 1; return; }  // finish this update
   if (S->itn - S->itn_mark >= STALL_WINDOW) {
     const bool flat = S->phibar > 0.5 * S->phibar_mark;
@@ -234,13 +261,45 @@ __global__ void k_minres_b_scalar(MinresState* S, const double* part, int nb) {
   if (S->itn >= S->maxit) { S->done = 2; S->status = S->phibar <= LOOSE_TOL * S->beta1 ? 4 : 2; }
 }
 
-// w_k = (v − oldeps·w_{k−2} − delta·w_{k−1})/gamma ; x += phi·w_k ; v ← (z − ⟨e,z⟩e)/β_{k+1}
-__global__ void __launch_bounds__(ADJ_NT) k_minres_c(AdjVecs V, MinresState* S) {
+// y ← y − ⟨e,y⟩e − (alfa/beta) r2 ; r1 ← r2 ; r2 ← y ; z = P r2 (into y) ; sums ⟨e,z⟩, ⟨r2,z⟩ (the
+// square of β_{k+1}: ⟨r2, z − e⟨e,z⟩⟩ = ⟨r2, z⟩ since r2 ⟂ e)
+__global__ void __launch_bounds__(ADJ_NT) k_minres_b(const AdjBand* __restrict__ bands, AdjGeom G) {
+  const AdjBand V = bands[blockIdx.y];
+  MinresState* S = V.S;
+  if (S->done) return;
+  const double c2 = S->alfa / S->beta, er0 = S->dot_ey_r, ei0 = S->dot_ey_i;
+  double d[4] = {0, 0, 0, 0};
+  for (int p = blockIdx.x * ADJ_NT + threadIdx.x; p < G.N; p += gridDim.x * ADJ_NT) {
+    const double s = prec_scale(p, G, V.k);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const size_t i = 2 * (size_t)p + c;
+      const double2 e = V.e[i], r2 = V.r2[i], y = sub_mul(V.y[i], er0, ei0, e);
+      const double2 yn = make_double2(y.x - c2 * r2.x, y.y - c2 * r2.y);
+      V.r1[i] = r2;
+      V.r2[i] = yn;
+      const double2 z = make_double2(yn.x * s, yn.y * s);
+      V.y[i] = z;
+      dot_acc(d[0], d[1], e, z);
+      dot_acc(d[2], d[3], yn, z);
+    }
+  }
+  if (!grid_sum4(d, V.part, V.ticket)) return;
+  S->dot_ez_r = d[0]; S->dot_ez_i = d[1];
+  minres_rotate(S, d[2]);
+}
+
+// w_k = (v − oldeps·w_{k−2} − delta·w_{k−1})/gamma ; x += phi·w_k ; v ← (z − ⟨e,z⟩e)/β_{k+1}; a solve
+// whose last update this was is then over
+__global__ void __launch_bounds__(ADJ_NT) k_minres_c(const AdjBand* __restrict__ bands, AdjGeom G) {
+  const AdjBand V = bands[blockIdx.y];
+  MinresState* S = V.S;
   if (S->done == 1) return;
   const double ig = 1.0 / S->gamma, oe = S->oldeps, de = S->delta, ph = S->phi;
   const bool next = S->done == 0 && S->beta > 0;
   const double ib = next ? 1.0 / S->beta : 0.0, er = S->dot_ez_r, ei = S->dot_ez_i;
-  for (long long i = blockIdx.x * (long long)ADJ_NT + threadIdx.x; i < V.n2; i += (long long)gridDim.x * ADJ_NT) {
+  const bool ends = S->done == 2;
+  for (int i = blockIdx.x * ADJ_NT + threadIdx.x; i < 2 * G.N; i += gridDim.x * ADJ_NT) {
     const double2 v = V.v[i], wa = V.w2[i], wb = V.w[i];
     const double2 wn = make_double2((v.x - oe * wa.x - de * wb.x) * ig, (v.y - oe * wa.y - de * wb.y) * ig);
     V.w2[i] = wb;
@@ -249,41 +308,28 @@ __global__ void __launch_bounds__(ADJ_NT) k_minres_c(AdjVecs V, MinresState* S) 
     x.x += ph * wn.x; x.y += ph * wn.y;
     V.x[i] = x;
     if (next) {
-      const double2 z = V.y[i], e = V.e[i];
-      V.v[i] = make_double2((z.x - (er * e.x - ei * e.y)) * ib, (z.y - (er * e.y + ei * e.x)) * ib);
+      const double2 z = sub_mul(V.y[i], er, ei, V.e[i]);
+      V.v[i] = make_double2(z.x * ib, z.y * ib);
     }
   }
-}
-__global__ void k_minres_finish(MinresState* S) {
-  if (threadIdx.x == 0 && blockIdx.x == 0 && S->done == 2) S->done = 1;
+  if (ends && last_block(V.ticket) && threadIdx.x == 0) { S->done = 1; S->active = 0; }
 }
 
-// λ ← λ − ⟨e,λ⟩e (two passes: partial dot, then update with the reduced value)
-__global__ void __launch_bounds__(ADJ_NT) k_dot_e(const double2* __restrict__ e, const double2* __restrict__ x,
-                                                  long long n, double* part) {
-  double r = 0, im = 0;
-  for (long long i = blockIdx.x * (long long)ADJ_NT + threadIdx.x; i < n; i += (long long)gridDim.x * ADJ_NT) {
-    const double2 a = e[i], b = x[i];
-    r += a.x * b.x + a.y * b.y; im += a.x * b.y - a.y * b.x;
-  }
-  block_reduce4(r, im, 0, 0, part);
+// t ← t − ⟨e,t⟩e for the right-hand sides (t = b) or the solutions (t = x): the sum, then the update
+// with it
+__global__ void __launch_bounds__(ADJ_NT) k_dot_e(const AdjBand* __restrict__ bands, AdjGeom G, int of_x) {
+  const AdjBand V = bands[blockIdx.y];
+  const double2* t = of_x ? V.x : V.b;
+  double d[4] = {0, 0, 0, 0};
+  for (int i = blockIdx.x * ADJ_NT + threadIdx.x; i < 2 * G.N; i += gridDim.x * ADJ_NT) dot_acc(d[0], d[1], V.e[i], t[i]);
+  if (!grid_sum4(d, V.part, V.ticket)) return;
+  V.S->dot_ey_r = d[0]; V.S->dot_ey_i = d[1];
 }
-__global__ void __launch_bounds__(ADJ_NT) k_sub_proj(const double2* __restrict__ e, double2* __restrict__ x, long long n,
-                                                     const double* part, int nb) {
-  __shared__ double cr, ci;
-  if (threadIdx.x == 0) {
-    double a = 0, b = 0;
-    for (int i = 0; i < nb; ++i) { a += part[4 * i]; b += part[4 * i + 1]; }
-    cr = a; ci = b;
-  }
-  __syncthreads();
-  for (long long i = blockIdx.x * (long long)ADJ_NT + threadIdx.x; i < n; i += (long long)gridDim.x * ADJ_NT) {
-    const double2 a = e[i];
-    double2 b = x[i];
-    b.x -= cr * a.x - ci * a.y;
-    b.y -= cr * a.y + ci * a.x;
-    x[i] = b;
-  }
+__global__ void __launch_bounds__(ADJ_NT) k_sub_proj(const AdjBand* __restrict__ bands, AdjGeom G, int of_x) {
+  const AdjBand V = bands[blockIdx.y];
+  double2* t = of_x ? V.x : V.b;
+  const double cr = V.S->dot_ey_r, ci = V.S->dot_ey_i;
+  for (int i = blockIdx.x * ADJ_NT + threadIdx.x; i < 2 * G.N; i += gridDim.x * ADJ_NT) t[i] = sub_mul(t[i], cr, ci, V.e[i]);
 }
 
 // k̄ₕ partials from ẽ = EC/N, λ̃e = ED/N (planar), h and λ (interleaved), basis at k
@@ -384,116 +430,146 @@ static int pullback_impl(omb_ctx* ctx, Problem& P, double omega, int nev, const 
   cudaStream_t st = ctx->stream;
   const long long N = (long long)P.N(), n2 = 2 * N;
   const bool periodic = P.Nz > 1;
-  const double inv_dz = periodic ? 1.0 / P.Dz : 0.0;  // (a 2D cell has Dz = 0)
-  // device buffers
-  DevBuf<double2> vecs, scr, ev, eb, lamv;
-  OMB_CU(vecs.alloc(8 * n2, st));   // x v w w2 r1 r2 y Av
-  OMB_CU(scr.alloc(6 * 3 * N, st)); // operator scratch ×2, copies ×2, E fields ×2
-  OMB_CU(ev.alloc(n2, st));
-  OMB_CU(eb.alloc(n2, st));
-  DevBuf<double> part, eib, kd, hpart, hred;
-  const int nb = ADJ_BLOCKS;
-  OMB_CU(part.alloc(4 * nb, st));
+  for (int b = 0; b < nev; ++b)
+    if (!(kmags[b] > 0) || !std::isfinite(kmags[b])) return fail(OMB_ERR_INVALID_ARG, "kmags must be finite and positive");
+  const AdjGeom G{(int)N, P.Nx, P.Ny, P.Nz, 1.0 / P.Dx, 1.0 / P.Dy, periodic ? 1.0 / P.Dz : 0.0, P.eps_mean};
+  const int rb = row_blocks(P.Nx, P.Ny) * P.Nz;  // HMₖH partials: row blocks of every slab
+  DevBuf<double> eib;
   OMB_CU(eib.alloc(6 * N, st));
   OMB_CU(eib.zero());
-  OMB_CU(kd.alloc(1, st));
-  const int rb = row_blocks(P.Nx, P.Ny) * P.Nz;  // HMₖH partials: row blocks of every slab
-  OMB_CU(hpart.alloc(2 * rb, st));
-  OMB_CU(hred.alloc(2, st));
-  DevBuf<MinresState> S;
-  OMB_CU(S.alloc(1, st));
-  double2* vb = vecs.p;
-  AdjVecs V{vb, vb + n2, vb + 2 * n2, vb + 3 * n2, vb + 4 * n2, vb + 5 * n2, vb + 6 * n2, vb + 7 * n2, ev.p,
-            n2, P.Nx, P.Ny, 1.0 / P.Dx, 1.0 / P.Dy, 0.0, P.eps_mean, P.Nz, inv_dz};
-  double2* SA = scr.p;              // D0 = fft(kx_tc h)
-  double2* SB = SA + 3 * N;         // Λd = fft(kx_tc λ)
-  double2* SC = SB + 3 * N;         // copies consumed by the D2E passes
-  double2* SD = SC + 3 * N;
-  double2* EC = SD + 3 * N;         // N·ẽ
-  double2* ED = EC + 3 * N;         // N·λ̃e
-  // operator units (FP64): M on v → Av; HMkH on h; H2D on h and λ; D2E on the copies
-  auto unit = [&](const double2* in, double2* out, double2* s) {
-    OpUnit<double> u = make_unit<double>(P);
-    u.in = in; u.out = out; u.scr = s; u.k_dev = kd.p; u.partial = hpart.p;
-    u.in_cs = n2; u.out_cs = n2; u.scr_cs = 3 * N; u.ncol = 1;
-    return u;
-  };
-  // (unit 6: HMₖH with the ẑ× action weighted by g_z/Λ, for ∂ω²/∂Λ)
-  OpUnit<double> hu[7] = {unit(V.v, V.Av, SC),   unit(ev.p, nullptr, SC), unit(ev.p, nullptr, SA),
-                          unit(V.x, nullptr, SB), unit(nullptr, EC, SC),   unit(nullptr, ED, SD),
-                          unit(ev.p, nullptr, SC)};
-  hu[4].out_cs = 3 * N;
-  hu[5].out_cs = 3 * N;
-  hu[6].zx_weight_gz = 1;
-  DevBuf<OpUnit<double>> du, dexp;
-  OMB_CU(du.alloc(7, st));
-  OMB_CU(cudaMemcpyAsync(du.p, hu, 7 * sizeof(OpUnit<double>), cudaMemcpyHostToDevice, st));
-  if (periodic) OMB_CU(dexp.alloc(P.Nz + 1, st));
-  const TwTables& tw = ctx->tw;
-  auto run = [&](OpKind kind, int u) -> cudaError_t {
-    return periodic ? launch_op3d<double>(kind, du.p + u, 1, P.Nx, P.Ny, P.Nz, 1, tw, dexp.p, st)
-                    : launch_op<double>(kind, du.p + u, 1, P.Nx, P.Ny, 1, tw, st);
-  };
-  // ⟨h|∂M̂|h⟩ with unit u (the device partials hold Re⟨h|kx_ct(…)⟩ = −HMₖH)
-  auto hmkh = [&](int u, double& out) -> cudaError_t {
-    cudaError_t e = run(OP_HMKH, u);
-    if (e != cudaSuccess) return e;
-    k_reduce_partials<<<1, 256, 0, st>>>(hpart.p, rb, 1, hred.p);
-    e = cudaGetLastError();
-    double hh[2];
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hh, hred.p, sizeof(hh), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    out = -hh[0];
-    return e;
-  };
   double wbar = 0.0, Lbar = 0.0;
-  for (int b = 0; b < nev; ++b) {
-    const double kb = kmags[b];
-    if (!(kb > 0) || !std::isfinite(kb)) return fail(OMB_ERR_INVALID_ARG, "kmags must be finite and positive");
-    V.k = kb;
-    OMB_CU(cudaMemcpyAsync(kd.p, &kb, sizeof(double), cudaMemcpyHostToDevice, st));
-    OMB_CU(cudaMemcpyAsync(ev.p, evecs + 4 * N * (size_t)b, n2 * sizeof(double2), cudaMemcpyHostToDevice, st));
-    // ∂ω²/∂k = 2⟨h|∂M̂/∂k|h⟩ and, on a periodic cell, ∂ω²/∂Λ = 2⟨h|∂M̂/∂Λ|h⟩ (period.jl:150-151)
-    double hk = 0, hL = 0;
-    OMB_CU(hmkh(1, hk));
-    const double dw2dk = 2.0 * hk;
-    if (!(dw2dk > 0) || !std::isfinite(dw2dk)) return fail(OMB_ERR_NAN, "non-positive ∂ω²/∂k in the pull-back");
-    if (periodic && L_bar) OMB_CU(hmkh(6, hL));
-    const double dw2dL = 2.0 * hL;
-    double Lbar_h = 0.0;
-    const double kb_bar = kbar ? kbar[b] : 0.0;
-    double kbar_h = 0.0;
-    const double* eb_host = evbar ? evbar + 4 * N * (size_t)b : nullptr;
-    bool have_eb = false;
-    if (eb_host)
-      for (long long i = 0; i < 2 * n2 && !have_eb; ++i) have_eb = eb_host[i] != 0.0;
-    // D0 = fft(kx_tc h) into SA
-    OMB_CU(run(OP_H2D, 2));
-    if (have_eb) {
-      // b = ē − h⟨h,ē⟩
-      OMB_CU(cudaMemcpyAsync(eb.p, eb_host, n2 * sizeof(double2), cudaMemcpyHostToDevice, st));
-      k_dot_e<<<nb, ADJ_NT, 0, st>>>(ev.p, eb.p, n2, part.p);
-      k_sub_proj<<<nb, ADJ_NT, 0, st>>>(ev.p, eb.p, n2, part.p, nb);
+  // The bands of a chunk run together: at a few hundred KB to a few MB per vector one band's launches
+  // leave most SMs idle.  A band holds 10 vectors and 6 planar fields (28·N complex numbers more than
+  // its inputs); a chunk is limited to 4 GiB of them.
+  const int chunk = (int)std::max<long long>(1, std::min<long long>(nev, ((long long)4 << 30) / (38 * N * (long long)sizeof(double2))));
+  for (int b0 = 0; b0 < nev; b0 += chunk) {
+    const int nb = std::min(chunk, nev - b0);
+    // bands with a field cotangent (the others need no adjoint solve)
+    std::vector<int> mb;  // MINRES index → band of the chunk
+    for (int j = 0; j < nb && evbar; ++j) {
+      const double* h = evbar + 4 * N * (size_t)(b0 + j);
+      bool any = false;
+      for (long long i = 0; i < 2 * n2 && !any; ++i) any = h[i] != 0.0;
+      if (any) mb.push_back(j);
+    }
+    const int nm = (int)mb.size();
+    DevBuf<double2> ev, vecs, scr;
+    DevBuf<double> kd, part, hpart, hred;
+    DevBuf<MinresState> S;
+    DevBuf<unsigned> tick;
+    DevBuf<AdjBand> dband;
+    OMB_CU(ev.alloc(n2 * nb, st));
+    OMB_CU(vecs.alloc(9 * n2 * nm, st));       // x v w w2 r1 r2 y Av b
+    OMB_CU(scr.alloc(6 * 3 * N * nb, st));
+    OMB_CU(kd.alloc(nb, st));
+    OMB_CU(hpart.alloc(2 * (size_t)rb * nb, st));
+    OMB_CU(hred.alloc(4 * (size_t)nb, st));
+    double2* SA = scr.p;                // D0 = fft(kx_tc h), per band of the chunk
+    double2* SB = SA + 3 * N * nb;      // Λd = fft(kx_tc λ)
+    double2* SC = SB + 3 * N * nb;      // copies consumed by the D2E passes, operator scratch
+    double2* SD = SC + 3 * N * nb;
+    double2* EC = SD + 3 * N * nb;      // N·ẽ
+    double2* ED = EC + 3 * N * nb;      // N·λ̃e
+    OMB_CU(cudaMemcpyAsync(kd.p, kmags + b0, nb * sizeof(double), cudaMemcpyHostToDevice, st));
+    OMB_CU(cudaMemcpyAsync(ev.p, evecs + 4 * N * (size_t)b0, n2 * nb * sizeof(double2), cudaMemcpyHostToDevice, st));
+    // operator units, kind by kind: HMₖH on h; HMₖH with the ẑ× action weighted by g_z/Λ (∂ω²/∂Λ); H2D on
+    // h; M̂ on v → Av; H2D on λ; D2E on the two copies
+    enum { U_HK = 0, U_HL = 1, U_D0 = 2, U_M = 3, U_LD = 4, U_EC = 5, U_ED = 6, U_KINDS = 7 };
+    std::vector<OpUnit<double>> hu(U_KINDS * (size_t)nb);
+    std::vector<AdjBand> hband(nm);
+    auto unit = [&](int j, const double2* in, double2* out, double2* s) {
+      OpUnit<double> u = make_unit<double>(P);
+      u.in = in; u.out = out; u.scr = s; u.k_dev = kd.p + j; u.partial = hpart.p + 2 * (size_t)rb * j;
+      u.in_cs = n2; u.out_cs = n2; u.scr_cs = 3 * N; u.ncol = 1;
+      return u;
+    };
+    if (nm > 0) {
+      OMB_CU(S.alloc(nm, st));
+      OMB_CU(tick.alloc(nm, st));
+      OMB_CU(tick.zero());
+      OMB_CU(dband.alloc(nm, st));
+      OMB_CU(part.alloc(4 * (size_t)ADJ_BLOCKS * nm, st));
+    }
+    for (int j = 0; j < nb; ++j) {
+      const double2* e = ev.p + n2 * j;
+      hu[U_HK * nb + j] = unit(j, e, nullptr, SC + 3 * N * j);
+      hu[U_HL * nb + j] = unit(j, e, nullptr, SC + 3 * N * j);
+      hu[U_HL * nb + j].zx_weight_gz = 1;
+      hu[U_D0 * nb + j] = unit(j, e, nullptr, SA + 3 * N * j);
+    }
+    for (int m = 0; m < nm; ++m) {
+      const int j = mb[m];
+      double2* v0 = vecs.p + 9 * n2 * m;
+      hband[m] = AdjBand{v0, v0 + n2, v0 + 2 * n2, v0 + 3 * n2, v0 + 4 * n2, v0 + 5 * n2, v0 + 6 * n2, v0 + 7 * n2,
+                         v0 + 8 * n2, ev.p + n2 * j, part.p + 4 * (size_t)ADJ_BLOCKS * m, tick.p + m, S.p + m,
+                         kmags[b0 + j]};
+      hu[U_M * nb + m] = unit(j, hband[m].v, hband[m].Av, SC + 3 * N * j);
+      hu[U_M * nb + m].ncol_dev = &S.p[m].active;
+      hu[U_LD * nb + m] = unit(j, hband[m].x, nullptr, SB + 3 * N * j);
+      hu[U_EC * nb + m] = unit(j, nullptr, EC + 3 * N * j, SC + 3 * N * j);
+      hu[U_ED * nb + m] = unit(j, nullptr, ED + 3 * N * j, SD + 3 * N * j);
+      hu[U_EC * nb + m].out_cs = hu[U_ED * nb + m].out_cs = 3 * N;
+    }
+    DevBuf<OpUnit<double>> du, dexp;
+    OMB_CU(du.alloc(hu.size(), st));
+    OMB_CU(cudaMemcpyAsync(du.p, hu.data(), hu.size() * sizeof(OpUnit<double>), cudaMemcpyHostToDevice, st));
+    if (periodic) OMB_CU(dexp.alloc((size_t)(P.Nz + 1) * nb, st));
+    const TwTables& tw = ctx->tw;
+    auto run = [&](OpKind kind, int u, int n) -> cudaError_t {
+      return periodic ? launch_op3d<double>(kind, du.p + u * nb, n, P.Nx, P.Ny, P.Nz, 1, tw, dexp.p, st)
+                      : launch_op<double>(kind, du.p + u * nb, n, P.Nx, P.Ny, 1, tw, st);
+    };
+    // ∂ω²/∂k = 2⟨h|∂M̂/∂k|h⟩ and, on a periodic cell, ∂ω²/∂Λ = 2⟨h|∂M̂/∂Λ|h⟩ (period.jl:150-151); the device
+    // partials hold Re⟨h|kx_ct(…)⟩ = −HMₖH
+    const bool want_L = periodic && L_bar;
+    std::vector<double> hk(4 * (size_t)nb, 0.0);
+    OMB_CU(run(OP_HMKH, U_HK, nb));
+    k_reduce_partials<<<nb, 256, 0, st>>>(hpart.p, rb, nb, hred.p);
+    OMB_CU(cudaGetLastError());
+    if (want_L) {
+      OMB_CU(run(OP_HMKH, U_HL, nb));
+      k_reduce_partials<<<nb, 256, 0, st>>>(hpart.p, rb, nb, hred.p + 2 * nb);
       OMB_CU(cudaGetLastError());
+    }
+    OMB_CU(cudaMemcpyAsync(hk.data(), hred.p, (want_L ? 4 : 2) * (size_t)nb * sizeof(double), cudaMemcpyDeviceToHost, st));
+    // D0 = fft(kx_tc h) into SA
+    OMB_CU(run(OP_H2D, U_D0, nb));
+    OMB_CU(cudaStreamSynchronize(st));
+    for (int j = 0; j < nb; ++j) {
+      const double dw2dk = -2.0 * hk[2 * j];
+      if (!(dw2dk > 0) || !std::isfinite(dw2dk)) return fail(OMB_ERR_NAN, "non-positive ∂ω²/∂k in the pull-back");
+    }
+    std::vector<double> kbar_h(nb, 0.0), Lbar_h(nb, 0.0);
+    if (iterations)
+      for (int j = 0; j < nb; ++j) iterations[b0 + j] = 0;
+    if (nm < nb) OMB_CU(cudaMemsetAsync(SB, 0, 3 * N * nb * sizeof(double2), st));
+    if (nm > 0) {
       MinresState s0{};
       s0.shift = omega * omega;
       s0.rtol = 1e-12;
       s0.maxit = std::max(4 * O.maxiter, 3000);
-      OMB_CU(cudaMemcpyAsync(S.p, &s0, sizeof(s0), cudaMemcpyHostToDevice, st));
-      k_minres_init<<<nb, ADJ_NT, 0, st>>>(V, eb.p, part.p);
-      k_minres_init_scalar<<<1, 32, 0, st>>>(S.p, part.p, nb);
-      k_minres_first_v<<<nb, ADJ_NT, 0, st>>>(V, S.p);
+      std::vector<MinresState> hs(nm, s0);
+      OMB_CU(cudaMemcpyAsync(S.p, hs.data(), nm * sizeof(MinresState), cudaMemcpyHostToDevice, st));
+      OMB_CU(cudaMemcpyAsync(dband.p, hband.data(), nm * sizeof(AdjBand), cudaMemcpyHostToDevice, st));
+      for (int m = 0; m < nm; ++m)
+        OMB_CU(cudaMemcpyAsync(hband[m].b, evbar + 4 * N * (size_t)(b0 + mb[m]), n2 * sizeof(double2),
+                               cudaMemcpyHostToDevice, st));
+      const AdjBand* D = dband.p;
+      const int nbx = (int)std::min<long long>(ADJ_BLOCKS, (N + ADJ_NT - 1) / ADJ_NT);
+      const dim3 gv(nbx, nm);
+      // b = ē − h⟨h,ē⟩
+      k_dot_e<<<gv, ADJ_NT, 0, st>>>(D, G, 0);
+      k_sub_proj<<<gv, ADJ_NT, 0, st>>>(D, G, 0);
+      k_minres_init<<<gv, ADJ_NT, 0, st>>>(D, G);
+      k_minres_first_v<<<gv, ADJ_NT, 0, st>>>(D, G);
       OMB_CU(cudaGetLastError());
-      // one MINRES iteration; 8 per graph replay, host checks the flag between replays
+      // one MINRES iteration of every band; 8 per graph replay, host checks the flags between replays
       auto iter = [&]() -> cudaError_t {
-        cudaError_t e = run(OP_M, 0);
+        cudaError_t e = run(OP_M, U_M, nm);
         if (e != cudaSuccess) return e;
-        k_minres_a<<<nb, ADJ_NT, 0, st>>>(V, S.p, part.p);
-        k_minres_a_scalar<<<1, 32, 0, st>>>(S.p, part.p, nb);
-        k_minres_b<<<nb, ADJ_NT, 0, st>>>(V, S.p, part.p);
-        k_minres_b_scalar<<<1, 32, 0, st>>>(S.p, part.p, nb);
-        k_minres_c<<<nb, ADJ_NT, 0, st>>>(V, S.p);
-        k_minres_finish<<<1, 32, 0, st>>>(S.p);
+        k_minres_a<<<gv, ADJ_NT, 0, st>>>(D, G);
+        k_minres_b<<<gv, ADJ_NT, 0, st>>>(D, G);
+        k_minres_c<<<gv, ADJ_NT, 0, st>>>(D, G);
         return cudaGetLastError();
       };
       OMB_CU(iter());  // eager once (sets kernel attributes outside the capture)
@@ -506,62 +582,73 @@ static int pullback_impl(omb_ctx* ctx, Problem& P, double omega, int nev, const 
       if (ce != cudaSuccess) { if (graph) cudaGraphDestroy(graph); return cuda_fail(ce, "MINRES capture"); }
       OMB_CU(ee);
       OMB_CU(cudaGraphInstantiate(&exec, graph, 0));
-      MinresState sh{};
       const int cap = s0.maxit / 8 + 2;
       for (int it = 0; it < cap; ++it) {
         cudaError_t e = cudaGraphLaunch(exec, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&sh, S.p, sizeof(sh), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(hs.data(), S.p, nm * sizeof(MinresState), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) { cudaGraphExecDestroy(exec); cudaGraphDestroy(graph); return cuda_fail(e, "MINRES"); }
-        if (sh.done) break;
+        bool all = true;
+        for (const MinresState& q : hs) all = all && q.done;
+        if (all) break;
       }
       cudaGraphExecDestroy(exec);
       cudaGraphDestroy(graph);
-      if (iterations) iterations[b] = sh.itn;
-      if (sh.status == 3) return fail(OMB_ERR_NAN, "MINRES breakdown in the adjoint solve");
-      if (sh.status != 1 && sh.status != 4) {
-        char msg[160];
-        snprintf(msg, sizeof msg, "adjoint MINRES did not converge (band %d: relative residual %.3g after %d iterations)",
-                 b, sh.beta1 > 0 ? sh.phibar / sh.beta1 : 0.0, sh.itn);
-        return fail(OMB_ERR_NOT_CONVERGED, msg);
+      for (int m = 0; m < nm; ++m) {
+        const MinresState& sh = hs[m];
+        const int b = b0 + mb[m];
+        if (iterations) iterations[b] = sh.itn;
+        if (sh.status == 3) return fail(OMB_ERR_NAN, "MINRES breakdown in the adjoint solve");
+        if (sh.status != 1 && sh.status != 4) {
+          char msg[160];
+          snprintf(msg, sizeof msg, "adjoint MINRES did not converge (band %d: relative residual %.3g after %d iterations)",
+                   b, sh.beta1 > 0 ? sh.phibar / sh.beta1 : 0.0, sh.itn);
+          return fail(OMB_ERR_NOT_CONVERGED, msg);
+        }
       }
       // λ ⟂ h (re-projection against round-off), then Λd = fft(kx_tc λ) into SB
-      k_dot_e<<<nb, ADJ_NT, 0, st>>>(ev.p, V.x, n2, part.p);
-      k_sub_proj<<<nb, ADJ_NT, 0, st>>>(ev.p, V.x, n2, part.p, nb);
+      k_dot_e<<<gv, ADJ_NT, 0, st>>>(D, G, 1);
+      k_sub_proj<<<gv, ADJ_NT, 0, st>>>(D, G, 1);
       OMB_CU(cudaGetLastError());
-      OMB_CU(run(OP_H2D, 3));
+      OMB_CU(run(OP_H2D, U_LD, nm));
       // ẽ·N and λ̃e·N through the D2E passes on copies (the passes work in place)
-      OMB_CU(cudaMemcpyAsync(SC, SA, 3 * N * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-      OMB_CU(cudaMemcpyAsync(SD, SB, 3 * N * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-      OMB_CU(run(OP_D2E, 4));
-      OMB_CU(run(OP_D2E, 5));
-      k_adj_kbar<<<nb, ADJ_NT, 0, st>>>(EC, ED, ev.p, V.x, P.Nx, P.Ny, P.Nz, 1.0 / P.Dx, 1.0 / P.Dy, inv_dz, kb,
-                                        part.p);
-      OMB_CU(cudaGetLastError());
-      std::vector<double> hp(4 * nb);
+      OMB_CU(cudaMemcpyAsync(SC, SA, 3 * N * nb * sizeof(double2), cudaMemcpyDeviceToDevice, st));
+      OMB_CU(cudaMemcpyAsync(SD, SB, 3 * N * nb * sizeof(double2), cudaMemcpyDeviceToDevice, st));
+      OMB_CU(run(OP_D2E, U_EC, nm));
+      OMB_CU(run(OP_D2E, U_ED, nm));
+      for (int m = 0; m < nm; ++m) {
+        const int j = mb[m];
+        k_adj_kbar<<<nbx, ADJ_NT, 0, st>>>(EC + 3 * N * j, ED + 3 * N * j, hband[m].e, hband[m].x, P.Nx, P.Ny, P.Nz,
+                                           G.inv_dx, G.inv_dy, G.inv_dz, kmags[b0 + j], hband[m].part);
+        OMB_CU(cudaGetLastError());
+      }
+      std::vector<double> hp(4 * (size_t)ADJ_BLOCKS * nm);
       OMB_CU(cudaMemcpyAsync(hp.data(), part.p, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
       OMB_CU(cudaStreamSynchronize(st));
-      double acc = 0, accL = 0;
-      for (int i = 0; i < nb; ++i) {
-        acc += hp[4 * i];
-        accL += hp[4 * i + 1];
+      for (int m = 0; m < nm; ++m) {
+        const double* q = hp.data() + 4 * (size_t)ADJ_BLOCKS * m;
+        double acc = 0, accL = 0;
+        for (int i = 0; i < nbx; ++i) {
+          acc += q[4 * i];
+          accL += q[4 * i + 1];
+        }
+        kbar_h[mb[m]] = -acc;
+        Lbar_h[mb[m]] = -accL;
       }
-      kbar_h = -acc;
-      Lbar_h = -accL;
-    } else {
-      if (iterations) iterations[b] = 0;
-      OMB_CU(cudaMemsetAsync(SB, 0, 3 * N * sizeof(double2), st));
     }
-    const double s = (kb_bar + kbar_h) / dw2dk;
-    k_adj_eibar<<<nb, ADJ_NT, 0, st>>>(SA, SB, N, s, eib.p);
-    OMB_CU(cudaGetLastError());
-    wbar += 2.0 * omega * s;
-    Lbar += Lbar_h + (kb_bar + kbar_h) * (-dw2dL / dw2dk);
+    for (int j = 0; j < nb; ++j) {
+      const double dw2dk = -2.0 * hk[2 * j], dw2dL = want_L ? -2.0 * hk[2 * (nb + j)] : 0.0;
+      const double kt = (kbar ? kbar[b0 + j] : 0.0) + kbar_h[j], s = kt / dw2dk;
+      k_adj_eibar<<<ADJ_BLOCKS, ADJ_NT, 0, st>>>(SA + 3 * N * j, SB + 3 * N * j, N, s, eib.p);
+      OMB_CU(cudaGetLastError());
+      wbar += 2.0 * omega * s;
+      Lbar += Lbar_h[j] + kt * (-dw2dL / dw2dk);
+    }
   }
   DevBuf<double> oei, oe;
   OMB_CU(oei.alloc(9 * N, st));
   if (eps_bar) OMB_CU(oe.alloc(9 * N, st));
-  k_adj_expand<<<nb, ADJ_NT, 0, st>>>(eib.p, P.e64.p, N, oei.p, eps_bar ? oe.p : nullptr);
+  k_adj_expand<<<ADJ_BLOCKS, ADJ_NT, 0, st>>>(eib.p, P.e64.p, N, oei.p, eps_bar ? oe.p : nullptr);
   OMB_CU(cudaGetLastError());
   OMB_CU(cudaMemcpyAsync(epsinv_bar, oei.p, 9 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (eps_bar) OMB_CU(cudaMemcpyAsync(eps_bar, oe.p, 9 * N * sizeof(double), cudaMemcpyDeviceToHost, st));

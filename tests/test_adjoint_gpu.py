@@ -116,3 +116,27 @@ def test_pullback_config1_rectangle(omb):
     wr, eir = O.solve_k_pullback(OMEGA0, ei, og, km, kv, kbar=kbar, evbar=evbar)
     assert np.isclose(wb, wr, rtol=1e-6)
     assert _rel(eib, eir) < 1e-5
+
+
+@pytest.mark.parametrize("nx,ny", [(8, 8), (24, 16), (40, 32), (320, 256)])
+def test_bands_solved_together_equal_bands_alone(omb, nx, ny):
+    """The adjoint solves of a pull-back run as rows of the same launches; every band's arithmetic is
+    the one it has alone (the same CTAs and summation order), so the sum of single-band pull-backs
+    differs from the joint one by the rounding of the final accumulation only.  Sizes: less than one
+    CTA of pixels, a remainder, a few CTAs, and more pixels than CTAs × threads."""
+    g = omb.Grid(6.0, 4.0, nx, ny)
+    ei = gaussian_epsinv(P_WG, Nx=nx, Ny=ny)
+    km, kv = omb.solve_k(OMEGA0, ei, g, omb.B200Solver(precision="fp64"), nev=3, k_tol=1e-11, eig_tol=1e-10)
+    rng = np.random.default_rng(nx)
+    ev = [rng.standard_normal(2 * g.N) + 1j * rng.standard_normal(2 * g.N) for _ in range(3)]
+    ev[1] = None
+    kb = [0.3, -0.7, 0.2]
+    wb, eib, info = omb.pullback(OMEGA0, ei, g, km, kv, kb, ev, return_info=True)
+    assert info["iterations"][1] == 0 and np.all(info["iterations"][[0, 2]] > 0)
+    w1, e1 = 0.0, 0.0
+    for j in range(3):
+        # (an all-None list is no cotangent)
+        w, e = omb.pullback(OMEGA0, ei, g, [km[j]], [kv[j]], [kb[j]], [ev[j]])
+        w1, e1 = w1 + w, e1 + e
+    assert np.isclose(wb, w1, rtol=1e-11, atol=0)
+    assert _rel(eib, e1) < 1e-11
