@@ -154,7 +154,7 @@ void big_free(void* p, cudaStream_t st) {
 }
 
 int row_blocks(int Nx, int Ny) {
-  const int rows = plan2_a(Nx) ? l2_rows(Nx) : rows_for(Nx);
+  const int rows = l2_rows(Nx);
   return (Ny + rows - 1) / rows;
 }
 
@@ -361,7 +361,8 @@ int upload_problem(omb_ctx* ctx, const omb_grid* g, const double* epsinv, Proble
   if (Nz > 1) {
     if (!fft_size_supported(Nz)) return fail(OMB_ERR_UNSUPPORTED, "unsupported Nz " + std::to_string(Nz));
     if (!(Dz > 0) || !std::isfinite(Dz)) return fail(OMB_ERR_INVALID_ARG, "the period Dz must be finite and positive");
-    if ((long long)Nz * row_blocks(g->Nx, g->Ny) > 512)
+    // (lines above 256 points are limited as if every row were a block)
+    if ((long long)Nz * (g->Nx > 256 ? g->Ny : row_blocks(g->Nx, g->Ny)) > 512)
       return fail(OMB_ERR_UNSUPPORTED, "Nz x row blocks of a slab above 512 (use fewer z slabs or rows)");
   } else if (Nz != 1) {
     return fail(OMB_ERR_INVALID_ARG, "Nz must be >= 1");

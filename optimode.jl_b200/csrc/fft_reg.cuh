@@ -17,7 +17,7 @@
 // reads of step 2 are both free of bank conflicts.
 //
 // The A- and B-point DFTs run entirely in registers: radix 2, 3, 4, 5, 8 butterflies
-// (fft_smem.cuh) and composites R = R1·R2 of them (the same factorisation with
+// (dft_small.cuh) and composites R = R1·R2 of them (the same factorisation with
 // compile-time indices and twiddle constants).  Twiddle constants are evaluated at
 // compile time from a Taylor series after reduction of the angle to [0, π/4].
 #pragma once
@@ -25,7 +25,7 @@
 #include <type_traits>
 #include <utility>
 
-#include "fft_smem.cuh"
+#include "dft_small.cuh"
 
 namespace omb {
 
@@ -95,10 +95,12 @@ template <int R, int E, bool INV, typename C> __device__ __forceinline__ C twc(C
 
 __host__ __device__ constexpr bool reg_dft_base(int R) { return R == 2 || R == 3 || R == 4 || R == 5 || R == 8; }
 __host__ __device__ constexpr bool reg_dft_ok(int R) {
-  return R == 1 || reg_dft_base(R) || R == 6 || R == 10 || R == 12 || R == 16;
+  return R == 1 || reg_dft_base(R) || R == 6 || R == 10 || R == 12 || R == 16 || R == 20 || R == 24 || R == 32;
 }
 // first factor of a composite register DFT
-__host__ __device__ constexpr int reg_split(int R) { return R == 16 ? 4 : R == 12 ? 4 : R == 10 ? 5 : 3; }
+__host__ __device__ constexpr int reg_split(int R) {
+  return R == 16 || R == 12 || R == 32 ? 4 : R == 10 || R == 20 ? 5 : 3;
+}
 
 // In-place DFT of R values held in registers, natural order in and out.
 template <int R, bool INV, typename C> __device__ __forceinline__ void dft_reg(C* v) {
@@ -133,11 +135,16 @@ template <int R, bool INV, typename C> __device__ __forceinline__ void dft_reg(C
 
 // ---- two-level plan ---------------------------------------------------------------------
 // A (first factor) for a line of length L, or 0 when L has no split into two register
-// DFT lengths ≤ 16.  Among valid splits the one with the smallest max(A, B) wins (fewest
-// idle threads), ties going to the larger A.
+// DFT lengths.  Among valid splits the one with the smallest max(A, B) wins (fewest
+// idle threads), ties going to the larger A.  Lines up to 256 split into lengths ≤ 16; 320, 384 and 512
+// into 20·16, 24·16 and 32·16, whose first factor is the one the passes transform one field component
+// at a time, so that a thread still holds at most 32 points of one component (64 registers in FP32,
+// 128 in FP64) or 16 points of three.  (Measured against shared-memory Stockham passes, which made
+// three round trips through shared memory per transform: an application to 4 columns of 16 512² cells
+// 1.89 → 0.67 ms in FP32 and 3.29 → 1.80 ms in FP64; 320² 0.57 → 0.28 and 1.00 → 0.67 ms.)
 __host__ __device__ constexpr int plan2_a(int L) {
   int best = 0, bestmax = 1 << 30;
-  for (int a = 16; a >= 2; --a) {
+  for (int a = 32; a >= 2; --a) {
     if (L % a != 0) continue;
     const int b = L / a;
     if (!reg_dft_ok(a) || !reg_dft_ok(b) || b < 2) continue;

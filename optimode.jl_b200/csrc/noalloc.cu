@@ -24,9 +24,8 @@
 //    one-thread kernel that receives them by value, on the caller's stream, ahead of the
 //    three passes; the field needs no clearing (the first pass writes every element the
 //    later passes read).
-//  * Lines that split into two register DFTs (every supported length up to 256) use the
-//    two-level register-FFT passes of omb_apply; 320, 384 and 512 use the shared-memory
-//    Stockham passes.  ε⁻¹ is read in the reference's (3, 3, Nx, Ny) layout.
+//  * The passes are the two-level register-FFT passes of omb_apply.  ε⁻¹ is read in the
+//    reference's (3, 3, Nx, Ny) layout.
 #include <cuda.h>
 
 #include <cmath>
@@ -155,33 +154,18 @@ template <typename K> static cudaError_t noalloc_launch(K kern, dim3 g, int nt, 
 
 template <int NX> static cudaError_t noalloc_rows(bool in, int Ny, int ncol, const OpUnit<float>* u,
                                                   const float2* tw, cudaStream_t st) {
-  if constexpr (plan2_a(NX) != 0) {  // two-level register FFT
-    constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
-    const size_t sm = (size_t)3 * G * l2_row_lstr<float2, NX>() * sizeof(float2);
-    const dim3 g((Ny + G - 1) / G, ncol, 1);
-    return in ? noalloc_launch(k_row_in2<float, NX, RI_KXTC, false>, g, NT, sm, st, u, tw)
-              : noalloc_launch(k_row_out2<float, NX, RO_KXCT, true>, g, NT, sm, st, u, tw);
-  } else {
-    constexpr int ROWS = rows_for(NX);
-    const size_t sm = (NX + 3 * ROWS * (NX + 1)) * sizeof(float2);
-    const dim3 g((Ny + ROWS - 1) / ROWS, ncol, 1);
-    return in ? noalloc_launch(k_row_in<float, NX, ROWS, NT_ROW, RI_KXTC, false>, g, NT_ROW, sm, st, u, tw)
-              : noalloc_launch(k_row_out<float, NX, ROWS, NT_ROW, RO_KXCT, true>, g, NT_ROW, sm, st, u, tw);
-  }
+  constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
+  const size_t sm = (size_t)3 * G * l2_row_lstr<float2, NX>() * sizeof(float2);
+  const dim3 g((Ny + G - 1) / G, ncol, 1);
+  return in ? noalloc_launch(k_row_in2<float, NX, RI_KXTC, false>, g, NT, sm, st, u, tw)
+            : noalloc_launch(k_row_out2<float, NX, RO_KXCT, true>, g, NT, sm, st, u, tw);
 }
 template <int NY> static cudaError_t noalloc_col(int Nx, int ncol, const OpUnit<float>* u, const float2* tw,
                                                  cudaStream_t st) {
-  if constexpr (plan2_a(NY) != 0) {  // two-level register FFT
-    constexpr int TX = l2_tx<float>(NY), NT = l2_col_threads<float>(NY);
-    const size_t sm = (size_t)3 * TX * l2_col_lstr<float2, NY, TX>() * sizeof(float2);
-    const dim3 g((Nx + TX - 1) / TX, ncol, 1);
-    return noalloc_launch(k_col2<float, NY, CS_FWD, PW_EPS9, CS_INV>, g, NT, sm, st, u, tw);
-  } else {
-    constexpr int TX = tx_for<float>(NY);
-    const size_t sm = (NY + 3 * TX * (NY + 1)) * sizeof(float2);
-    const dim3 g((Nx + TX - 1) / TX, ncol, 1);
-    return noalloc_launch(k_col<float, NY, TX, NT_COL, CS_FWD, PW_EPS9, CS_INV>, g, NT_COL, sm, st, u, tw);
-  }
+  constexpr int TX = l2_tx<float>(NY), NT = l2_col_threads<float>(NY);
+  const size_t sm = (size_t)3 * TX * l2_col_lstr<float2, NY, TX>() * sizeof(float2);
+  const dim3 g((Nx + TX - 1) / TX, ncol, 1);
+  return noalloc_launch(k_col2<float, NY, CS_FWD, PW_EPS9, CS_INV>, g, NT, sm, st, u, tw);
 }
 
 }  // namespace omb

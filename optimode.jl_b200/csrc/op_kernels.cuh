@@ -1,11 +1,12 @@
-// Fused plane-wave Helmholtz operator passes (sm_100a).
+// Fused plane-wave Helmholtz operator passes (sm_100a): the units they work on and their modes (the
+// kernels are in op_kernels_2l.cuh, op_kernels_split.cuh and op_cluster.cuh).
 //
 // One operator application M̂(k)H = kx_ct · (1/N)·bfft · ε⁻¹ · fft · kx_tc H
 // (reference: _M!, lib/MaxwellEigenmodes/src/maxwell.jl:471-481) runs as three passes:
 //
 //   row_in  : per grid row, regenerate (mag, m̂, n̂) from (k, gx, gy) in registers, form
-//             the 3-component field (kx_tc, kxinv_tc or zx_tc), FFT along x in shared
-//             memory, store planar to the scratch field (stays in L2 between passes);
+//             the 3-component field (kx_tc, kxinv_tc or zx_tc), FFT along x,
+//             store planar to the scratch field (stays in L2 between passes);
 //   col     : per tile of TX adjacent columns, FFT along y, per-pixel 3×3 ε⁻¹ contraction
 //             (6 unique entries: float4 + float2 loads) or ε_ave scaling, FFT back along y,
 //             in place;
@@ -21,7 +22,7 @@
 // (xx, yy, zz, xy) + (xz, yz) per pixel.
 #pragma once
 
-#include "fft_smem.cuh"
+#include "dft_small.cuh"
 
 namespace omb {
 
@@ -70,234 +71,6 @@ template <typename T> __device__ __forceinline__ int unit_ncol(const OpUnit<T>& 
 }
 template <typename T> __device__ __forceinline__ int unit_col0(const OpUnit<T>& U) {
   return U.col0_dev ? *U.col0_dev : 0;
-}
-
-template <typename C> __device__ __forceinline__ void load_tw(C* tw, const C* tw_g, int L) {
-  for (int i = threadIdx.x; i < L; i += blockDim.x) tw[i] = tw_g[i];
-}
-
-// ------------------------------------------------------------------------------------
-// row_in: prologue + FFT along x.  Grid: (ceil(Ny/ROWS), max columns, units).
-template <typename T, int NX, int ROWS, int NT, int MODE, bool INV>
-__global__ void __launch_bounds__(NT) k_row_in(const OpUnit<T>* __restrict__ units,
-                                               const cplx<T>* __restrict__ tw_g) {
-  using C = cplx<T>;
-  constexpr int LS = NX + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tw = reinterpret_cast<C*>(smem_raw);
-  C* s = tw + NX;
-  const OpUnit<T>& U = units[blockIdx.z];
-  const int col = blockIdx.y;
-  if (col >= unit_ncol(U)) return;
-  const int Ny = U.Ny;
-  const int row0 = blockIdx.x * ROWS;
-  if (row0 >= Ny) return;
-  const size_t N = U.comp_stride ? (size_t)U.comp_stride : (size_t)NX * Ny;
-  load_tw(tw, tw_g, NX);
-  const T k = (T)(*U.k_dev - U.kz_shift);
-  const C* __restrict__ H = U.in + (size_t)(col + unit_col0(U)) * U.in_cs;
-#pragma unroll
-  for (int q = threadIdx.x; q < ROWS * NX; q += NT) {
-    const int r = q / NX, ix = q - r * NX, iy = row0 + r;
-    C d0 = mk<C>(0, 0), d1 = d0, d2 = d0;
-    if (iy < Ny) {
-      const size_t p = ix + (size_t)NX * iy;
-      if constexpr (MODE == RI_LOAD3) {
-        d0 = H[p]; d1 = H[N + p]; d2 = H[2 * N + p];
-      } else {
-        C h1 = H[2 * p], h2 = H[2 * p + 1];
-        const Basis<T> b = basis_at<T>(k, T(freq_index(ix, NX)) * U.inv_dx, T(freq_index(iy, Ny)) * U.inv_dy);
-        if constexpr (MODE == RI_KXTC) {
-          const T s_ = -b.mag;
-          d0 = (h1 * b.nx - h2 * b.mx) * s_;
-          d1 = (h1 * b.ny - h2 * b.my) * s_;
-          d2 = h2 * (-b.mz * s_);
-        } else if constexpr (MODE == RI_KXINV) {
-          const T s_ = T(1) / b.mag;
-          d0 = (h1 * b.nx - h2 * b.mx) * s_;
-          d1 = (h1 * b.ny - h2 * b.my) * s_;
-          d2 = h2 * (-b.mz * s_);
-        } else if constexpr (MODE == RI_HCART) {  // Cartesian H = h1 m̂ + h2 n̂
-          d0 = h1 * b.mx + h2 * b.nx;
-          d1 = h1 * b.my + h2 * b.ny;
-          d2 = h1 * b.mz;
-        } else {  // RI_ZXTC: ẑ × (h1 m̂ + h2 n̂)
-          d0 = (h1 * b.my + h2 * b.ny) * T(-1);
-          d1 = h1 * b.mx + h2 * b.nx;
-          if (U.zx_weight_gz) {
-            const T wz = (T)(U.kz_shift * U.inv_dz);
-            d0 = d0 * wz;
-            d1 = d1 * wz;
-          }
-        }
-      }
-    }
-    s[(0 * ROWS + r) * LS + ix] = d0;
-    s[(1 * ROWS + r) * LS + ix] = d1;
-    s[(2 * ROWS + r) * LS + ix] = d2;
-  }
-  __syncthreads();
-  fft_lines<C, NX, INV, 3 * ROWS, NT>(s, LS, tw);
-  C* __restrict__ D = U.scr + (size_t)col * U.scr_cs;
-#pragma unroll
-  for (int q = threadIdx.x; q < ROWS * NX; q += NT) {
-    const int r = q / NX, ix = q - r * NX, iy = row0 + r;
-    if (iy < Ny) {
-      const size_t p = ix + (size_t)NX * iy;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) D[c * N + p] = s[(c * ROWS + r) * LS + ix];
-    }
-  }
-}
-
-// ------------------------------------------------------------------------------------
-// col: FFT along y, pointwise, FFT along y (each optional), in place on the scratch.
-// Grid: (ceil(Nx/TX), max columns, units).
-template <typename T, int NY, int TX, int NT, int S1, int PW, int S2>
-__global__ void __launch_bounds__(NT) k_col(const OpUnit<T>* __restrict__ units,
-                                            const cplx<T>* __restrict__ tw_g) {
-  using C = cplx<T>;
-  constexpr int LS = NY + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tw = reinterpret_cast<C*>(smem_raw);
-  C* s = tw + NY;
-  const OpUnit<T>& U = units[blockIdx.z];
-  const int col = blockIdx.y;
-  if (col >= unit_ncol(U)) return;
-  const int Nx = U.Nx;
-  const int ix0 = blockIdx.x * TX;
-  if (ix0 >= Nx) return;
-  const size_t N = U.comp_stride ? (size_t)U.comp_stride : (size_t)Nx * NY;
-  load_tw(tw, tw_g, NY);
-  C* __restrict__ D = U.scr + (size_t)col * U.scr_cs;
-#pragma unroll
-  for (int q = threadIdx.x; q < 3 * NY * TX; q += NT) {
-    const int t = q % TX, rest = q / TX, iy = rest % NY, c = rest / NY, ix = ix0 + t;
-    s[(c * TX + t) * LS + iy] = (ix < Nx) ? D[c * N + (size_t)iy * Nx + ix] : mk<C>(0, 0);
-  }
-  __syncthreads();
-  if constexpr (S1 != CS_NONE) fft_lines<C, NY, S1 == CS_INV, 3 * TX, NT>(s, LS, tw);
-  if constexpr (PW != PW_NONE) {
-#pragma unroll
-    for (int q = threadIdx.x; q < TX * NY; q += NT) {
-      const int t = q % TX, iy = q / TX, ix = ix0 + t;
-      if (ix < Nx) {
-        const size_t p = ix + (size_t)Nx * iy;
-        C* a0 = &s[(0 * TX + t) * LS + iy];
-        C* a1 = &s[(1 * TX + t) * LS + iy];
-        C* a2 = &s[(2 * TX + t) * LS + iy];
-        const C d0 = *a0, d1 = *a1, d2 = *a2;
-        if constexpr (PW == PW_EPS || PW == PW_EPS9) {
-          T e[6];
-          if constexpr (PW == PW_EPS) {
-            load_eps<T>(U, p, e);
-          } else {  // the reference's (3, 3, Nx, Ny) column-major layout, 9 entries per pixel
-            const T* m = U.e9 + 9 * p;
-            e[0] = m[0]; e[1] = m[4]; e[2] = m[8];
-            e[3] = T(0.5) * (m[1] + m[3]); e[4] = T(0.5) * (m[2] + m[6]); e[5] = T(0.5) * (m[5] + m[7]);
-          }
-          // symmetric ε⁻¹ = [[xx, xy, xz], [xy, yy, yz], [xz, yz, zz]]
-          *a0 = d0 * e[0] + d1 * e[3] + d2 * e[4];
-          *a1 = d0 * e[3] + d1 * e[1] + d2 * e[5];
-          *a2 = d0 * e[4] + d1 * e[5] + d2 * e[2];
-        } else {
-          const T w = U.eave[p];
-          *a0 = d0 * w; *a1 = d1 * w; *a2 = d2 * w;
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if constexpr (S2 != CS_NONE) fft_lines<C, NY, S2 == CS_INV, 3 * TX, NT>(s, LS, tw);
-#pragma unroll
-  for (int q = threadIdx.x; q < 3 * NY * TX; q += NT) {
-    const int t = q % TX, rest = q / TX, iy = rest % NY, c = rest / NY, ix = ix0 + t;
-    if (ix < Nx) D[c * N + (size_t)iy * Nx + ix] = s[(c * TX + t) * LS + iy];
-  }
-}
-
-// ------------------------------------------------------------------------------------
-// row_out: FFT along x + epilogue.  Grid: (ceil(Ny/ROWS), max columns, units).
-template <typename T, int NX, int ROWS, int NT, int MODE, bool INV>
-__global__ void __launch_bounds__(NT) k_row_out(const OpUnit<T>* __restrict__ units,
-                                                const cplx<T>* __restrict__ tw_g) {
-  using C = cplx<T>;
-  constexpr int LS = NX + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tw = reinterpret_cast<C*>(smem_raw);
-  C* s = tw + NX;
-  __shared__ double red[2][NT / 32];
-  const OpUnit<T>& U = units[blockIdx.z];
-  const int col = blockIdx.y;
-  if (col >= unit_ncol(U)) return;
-  const int Ny = U.Ny;
-  const int row0 = blockIdx.x * ROWS;
-  if (row0 >= Ny) return;
-  const size_t N = U.comp_stride ? (size_t)U.comp_stride : (size_t)NX * Ny;
-  load_tw(tw, tw_g, NX);
-  const C* __restrict__ D = U.scr + (size_t)col * U.scr_cs;
-#pragma unroll
-  for (int q = threadIdx.x; q < ROWS * NX; q += NT) {
-    const int r = q / NX, ix = q - r * NX, iy = row0 + r;
-    const bool ok = iy < Ny;
-    const size_t p = ix + (size_t)NX * iy;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) s[(c * ROWS + r) * LS + ix] = ok ? D[c * N + p] : mk<C>(0, 0);
-  }
-  __syncthreads();
-  fft_lines<C, NX, INV, 3 * ROWS, NT>(s, LS, tw);
-  const T k = (T)(*U.k_dev - U.kz_shift);
-  const T sN = T(1) / T(N);
-  const int c0 = unit_col0(U);
-  C* __restrict__ O = U.out + (size_t)(col + c0) * U.out_cs;
-  double accr = 0.0, acci = 0.0;
-#pragma unroll
-  for (int q = threadIdx.x; q < ROWS * NX; q += NT) {
-    const int r = q / NX, ix = q - r * NX, iy = row0 + r;
-    if (iy >= Ny) continue;
-    const size_t p = ix + (size_t)NX * iy;
-    const C e0 = s[(0 * ROWS + r) * LS + ix], e1 = s[(1 * ROWS + r) * LS + ix], e2 = s[(2 * ROWS + r) * LS + ix];
-    if constexpr (MODE == RO_STORE3) {
-      O[p] = e0; O[N + p] = e1; O[2 * N + p] = e2;
-    } else {
-      const Basis<T> b = basis_at<T>(k, T(freq_index(ix, NX)) * U.inv_dx, T(freq_index(iy, Ny)) * U.inv_dy);
-      const C en = e0 * b.nx + e1 * b.ny;                 // e·n̂ (n̂_z = 0)
-      const C em = e0 * b.mx + e1 * b.my + e2 * b.mz;     // e·m̂
-      C h1, h2;
-      if constexpr (MODE == RO_KXINVCT) {
-        const T sc = sN / b.mag;
-        h1 = en * sc; h2 = em * (-sc);
-      } else {
-        const T sc = b.mag * sN;
-        h1 = en * (-sc); h2 = em * sc;
-      }
-      if constexpr (MODE == RO_KXCT_DOT) {
-        const C* Hin = U.in + (size_t)(col + c0) * U.in_cs;
-        const C g1 = Hin[2 * p], g2 = Hin[2 * p + 1];
-        // ⟨H_in, out⟩ = Σ conj(H_in)·out
-        accr += (double)g1.x * h1.x + (double)g1.y * h1.y + (double)g2.x * h2.x + (double)g2.y * h2.y;
-        acci += (double)g1.x * h1.y - (double)g1.y * h1.x + (double)g2.x * h2.y - (double)g2.y * h2.x;
-      } else {
-        O[2 * p] = h1; O[2 * p + 1] = h2;
-      }
-    }
-  }
-  if constexpr (MODE == RO_KXCT_DOT) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      accr += __shfl_xor_sync(0xffffffffu, accr, o);
-      acci += __shfl_xor_sync(0xffffffffu, acci, o);
-    }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) { red[0][w] = accr; red[1][w] = acci; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double sr = 0, si = 0;
-      for (int i = 0; i < NT / 32; ++i) { sr += red[0][i]; si += red[1][i]; }
-      double* P = U.partial + 2 * ((size_t)col * U.part_stride + blockIdx.x);
-      P[0] = sr; P[1] = si;
-    }
-  }
 }
 
 }  // namespace omb

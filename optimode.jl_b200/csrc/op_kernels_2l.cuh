@@ -1,6 +1,4 @@
-// Operator passes on the two-level register FFT (fft_reg.cuh) for line lengths that split
-// into two register DFTs (≤ 256 here); longer lines use the Stockham passes of
-// op_kernels.cuh.  Same three passes, modes, layouts and results as those kernels:
+// Operator passes on the two-level register FFT (fft_reg.cuh):
 //
 //   row_in  : G grid rows per CTA; global H → prologue → step 1 (A-point DFTs) → padded
 //             block → step 2 (B-point DFTs) → planar scratch, coalesced along x;
@@ -43,7 +41,9 @@ __host__ __device__ constexpr int l2_rows(int NX) {
 }
 __host__ __device__ constexpr int l2_row_threads(int NX, int G) { return (G * plan2_max(NX) + 31) / 32 * 32; }
 __host__ __device__ constexpr int l2_row_threads(int NX) { return l2_row_threads(NX, l2_rows(NX)); }
-template <typename T> __host__ __device__ constexpr int l2_tx(int NY) { return 8; }
+// Columns per CTA of the column pass: 8 (64-byte row segments in FP32); FP64 lines above 256 points
+// take 4, whose 105 KB block leaves room for a second CTA.
+template <typename T> __host__ __device__ constexpr int l2_tx(int NY) { return sizeof(T) == 8 && NY > 256 ? 4 : 8; }
 __host__ __device__ constexpr int l2_col_threads_tx(int NY, int TX) { return (TX * plan2_max(NY) + 31) / 32 * 32; }
 template <typename T> __host__ __device__ constexpr int l2_col_threads(int NY) {
   return l2_col_threads_tx(NY, l2_tx<T>(NY));
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(l2_row_threads(NX, G)) k_row_in2(const OpUnit<
   using C = cplx<T>;
   constexpr int A = plan2_a(NX), B = NX / A, NT = l2_row_threads(NX, G);
   constexpr int LS = l2_row_lstr<C, NX>();
-  constexpr bool REG3 = sizeof(T) == 4;
+  constexpr bool REG3 = sizeof(T) == 4 && A <= 16;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* blk = reinterpret_cast<C*>(smem_raw);  // [3][G][LS]
   const OpUnit<T>& U = units[blockIdx.z];
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(l2_row_threads(NX, G)) k_row_out2(const OpUnit
   using C = cplx<T>;
   constexpr int A = plan2_a(NX), B = NX / A, NT = l2_row_threads(NX, G);
   constexpr int LS = l2_row_lstr<C, NX>();
-  constexpr bool REG3 = sizeof(T) == 4;
+  constexpr bool REG3 = sizeof(T) == 4 && A <= 16;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* blk = reinterpret_cast<C*>(smem_raw);  // [3][G][LS]
   __shared__ double red[2][NT / 32 + 1];

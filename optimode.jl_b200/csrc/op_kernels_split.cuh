@@ -1,4 +1,4 @@
-// Component-parallel operator passes for two-level lines (≤ 256 points): FP32 row and
+// Component-parallel operator passes for two-level lines: FP32 row and
 // column passes (tile variants) and the FP64 row passes.
 //
 // The same transforms, modes, layouts and results as k_row_in2 / k_col2 / k_row_out2
@@ -23,14 +23,15 @@ __host__ __device__ constexpr int sp_col_threads(int NY, int TX) { return (3 * T
 // CTAs per SM the register budget is set for (the 52 KB FP32 block allows four; an FP64 row
 // block is twice as large and its A or B complex doubles need ≈80 registers)
 __host__ __device__ constexpr int sp_min_blocks(int nt) { return nt <= 384 ? 3 : (nt <= 512 ? 2 : 1); }
-template <typename T> __host__ __device__ constexpr int sp_row_min_blocks(int nt) {
-  return sizeof(T) == 4 ? sp_min_blocks(nt) : (nt <= 512 ? 2 : 1);
+// (lines above 256 points hold up to 32 of a component: two FP32 CTAs, one FP64)
+template <typename T> __host__ __device__ constexpr int sp_row_min_blocks(int nt, int NX) {
+  return NX > 256 ? (sizeof(T) == 4 ? 2 : 1) : (sizeof(T) == 4 ? sp_min_blocks(nt) : (nt <= 512 ? 2 : 1));
 }
 
 // ------------------------------------------------------------------------------------
 // row_in.  Grid: (ceil(Ny/G), max columns, units); sp_row_threads(NX, G) threads.
 template <typename T, int NX, int MODE, bool INV, int G>
-__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G)))
+__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G), NX))
     k_row_in_sp(const OpUnit<T>* __restrict__ units, const cplx<T>* __restrict__ tw_g) {
   using C = cplx<T>;
   constexpr int A = plan2_a(NX), B = NX / A, NT = sp_row_threads(NX, G);
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(sp_col_threads(NY, TX), MINB)
 // ------------------------------------------------------------------------------------
 // row_out.  Grid: (ceil(Ny/G), max columns, units); sp_row_threads(NX, G) threads.
 template <typename T, int NX, int MODE, bool INV, int G>
-__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G)))
+__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G), NX))
     k_row_out_sp(const OpUnit<T>* __restrict__ units, const cplx<T>* __restrict__ tw_g) {
   using C = cplx<T>;
   constexpr int A = plan2_a(NX), B = NX / A, NT = sp_row_threads(NX, G);

@@ -14,15 +14,10 @@ namespace omb {
 #define OMB_FFT_SIZES(X) X(8) X(12) X(16) X(20) X(24) X(32) X(40) X(48) X(64) X(80) X(96) \
   X(128) X(160) X(192) X(256) X(320) X(384) X(512)
 
-// Launch shape policy.  Row passes: NT_ROW threads, ROWS grid rows per CTA (≈512 pixels).
-// Column pass: NT_COL threads, TX adjacent columns per CTA (8 for coalesced row segments,
-// 4 for FP64 above 256 points to stay inside the shared-memory budget).
-constexpr int NT_ROW = 128;
-constexpr int NT_COL = 256;
-__host__ __device__ constexpr int rows_for(int NX) { return NX >= 512 ? 1 : 512 / NX; }
-template <typename T> __host__ __device__ constexpr int tx_for(int NY) {
-  return (NY <= 256) ? 8 : (sizeof(T) == 4 ? 8 : 4);
-}
+// every supported length has a two-level plan
+#define OMB_CASE(L) static_assert(plan2_a(L) != 0, "no two-level plan");
+OMB_FFT_SIZES(OMB_CASE)
+#undef OMB_CASE
 
 template <typename T>
 using PassKernel = void (*)(const OpUnit<T>*, const cplx<T>*);
@@ -108,7 +103,7 @@ static cudaError_t col_sp(const OpUnit<float>* u, int nunits, int Nx, int maxcol
 template <typename T, int NX>
 static cudaError_t row_in_nx(int mode, const OpUnit<T>* u, int nunits, int Ny, int maxcol,
                              const cplx<T>* tw, cudaStream_t st, int gv = 1) {
-  if constexpr (plan2_a(NX) != 0 && sizeof(T) == 4) {
+  if constexpr (sizeof(T) == 4) {
     if (mode == RI_KXTC && (gv == 3 || gv == 4))
       return row_in_sp<NX, RI_KXTC, false>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Ny, maxcol,
                                            reinterpret_cast<const float2*>(tw), st);
@@ -116,40 +111,26 @@ static cudaError_t row_in_nx(int mode, const OpUnit<T>* u, int nunits, int Ny, i
       return gv == 0 ? row_in_g<T, NX, row_g_variant<NX>(0), RI_KXTC, false>(u, nunits, Ny, maxcol, tw, st)
                      : row_in_g<T, NX, row_g_variant<NX>(2), RI_KXTC, false>(u, nunits, Ny, maxcol, tw, st);
   }
-  if constexpr (plan2_a(NX) != 0 && sizeof(T) == 8) {
+  if constexpr (sizeof(T) == 8) {
     if (FP64_ROW_SPLIT && mode == RI_KXTC) return row_in_sp<NX, RI_KXTC, false, T>(u, nunits, Ny, maxcol, tw, st);
   }
-  if constexpr (plan2_a(NX) != 0) {  // two-level register FFT
-    constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
-    const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
-    const dim3 g((Ny + G - 1) / G, maxcol, nunits);
-    switch (mode) {
-      case RI_KXTC: return launch_pass<T>(k_row_in2<T, NX, RI_KXTC, false>, g, NT, sm, st, u, tw);
-      case RI_KXINV: return launch_pass<T>(k_row_in2<T, NX, RI_KXINV, true>, g, NT, sm, st, u, tw);
-      case RI_ZXTC: return launch_pass<T>(k_row_in2<T, NX, RI_ZXTC, false>, g, NT, sm, st, u, tw);
-      case RI_HCART: return launch_pass<T>(k_row_in2<T, NX, RI_HCART, false>, g, NT, sm, st, u, tw);
-      case RI_LOAD3: return launch_pass<T>(k_row_in2<T, NX, RI_LOAD3, true>, g, NT, sm, st, u, tw);
-      default: return cudaErrorInvalidValue;
-    }
-  } else {
-    constexpr int ROWS = rows_for(NX);
-    const size_t sm = (NX + 3 * ROWS * (NX + 1)) * sizeof(cplx<T>);
-    const dim3 g((Ny + ROWS - 1) / ROWS, maxcol, nunits);
-    switch (mode) {
-      case RI_KXTC: return launch_pass<T>(k_row_in<T, NX, ROWS, NT_ROW, RI_KXTC, false>, g, NT_ROW, sm, st, u, tw);
-      case RI_KXINV: return launch_pass<T>(k_row_in<T, NX, ROWS, NT_ROW, RI_KXINV, true>, g, NT_ROW, sm, st, u, tw);
-      case RI_ZXTC: return launch_pass<T>(k_row_in<T, NX, ROWS, NT_ROW, RI_ZXTC, false>, g, NT_ROW, sm, st, u, tw);
-      case RI_HCART: return launch_pass<T>(k_row_in<T, NX, ROWS, NT_ROW, RI_HCART, false>, g, NT_ROW, sm, st, u, tw);
-      case RI_LOAD3: return launch_pass<T>(k_row_in<T, NX, ROWS, NT_ROW, RI_LOAD3, true>, g, NT_ROW, sm, st, u, tw);
-      default: return cudaErrorInvalidValue;
-    }
+  constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
+  const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
+  const dim3 g((Ny + G - 1) / G, maxcol, nunits);
+  switch (mode) {
+    case RI_KXTC: return launch_pass<T>(k_row_in2<T, NX, RI_KXTC, false>, g, NT, sm, st, u, tw);
+    case RI_KXINV: return launch_pass<T>(k_row_in2<T, NX, RI_KXINV, true>, g, NT, sm, st, u, tw);
+    case RI_ZXTC: return launch_pass<T>(k_row_in2<T, NX, RI_ZXTC, false>, g, NT, sm, st, u, tw);
+    case RI_HCART: return launch_pass<T>(k_row_in2<T, NX, RI_HCART, false>, g, NT, sm, st, u, tw);
+    case RI_LOAD3: return launch_pass<T>(k_row_in2<T, NX, RI_LOAD3, true>, g, NT, sm, st, u, tw);
+    default: return cudaErrorInvalidValue;
   }
 }
 
 template <typename T, int NX>
 static cudaError_t row_out_nx(int mode, const OpUnit<T>* u, int nunits, int Ny, int maxcol,
                               const cplx<T>* tw, cudaStream_t st, int gv = 1) {
-  if constexpr (plan2_a(NX) != 0 && sizeof(T) == 4) {
+  if constexpr (sizeof(T) == 4) {
     // (the dot-product mode keeps the default rows: its partial sums are laid out per row block)
     if (mode == RO_KXCT && gv == 3)
       return row_out_nx<T, NX>(mode, u, nunits, Ny, maxcol, tw, st, 1);
@@ -163,31 +144,18 @@ static cudaError_t row_out_nx(int mode, const OpUnit<T>* u, int nunits, int Ny, 
       return gv == 0 ? row_out_g<T, NX, row_g_variant<NX>(0), RO_KXCT, true>(u, nunits, Ny, maxcol, tw, st)
                      : row_out_g<T, NX, row_g_variant<NX>(2), RO_KXCT, true>(u, nunits, Ny, maxcol, tw, st);
   }
-  if constexpr (plan2_a(NX) != 0 && sizeof(T) == 8) {
+  if constexpr (sizeof(T) == 8) {
     if (FP64_ROW_SPLIT && mode == RO_KXCT) return row_out_sp<NX, RO_KXCT, true, T>(u, nunits, Ny, maxcol, tw, st);
   }
-  if constexpr (plan2_a(NX) != 0) {  // two-level register FFT
-    constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
-    const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
-    const dim3 g((Ny + G - 1) / G, maxcol, nunits);
-    switch (mode) {
-      case RO_KXCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT, true>, g, NT, sm, st, u, tw);
-      case RO_KXINVCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXINVCT, false>, g, NT, sm, st, u, tw);
-      case RO_STORE3: return launch_pass<T>(k_row_out2<T, NX, RO_STORE3, true>, g, NT, sm, st, u, tw);
-      case RO_KXCT_DOT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT_DOT, true>, g, NT, sm, st, u, tw);
-      default: return cudaErrorInvalidValue;
-    }
-  } else {
-    constexpr int ROWS = rows_for(NX);
-    const size_t sm = (NX + 3 * ROWS * (NX + 1)) * sizeof(cplx<T>);
-    const dim3 g((Ny + ROWS - 1) / ROWS, maxcol, nunits);
-    switch (mode) {
-      case RO_KXCT: return launch_pass<T>(k_row_out<T, NX, ROWS, NT_ROW, RO_KXCT, true>, g, NT_ROW, sm, st, u, tw);
-      case RO_KXINVCT: return launch_pass<T>(k_row_out<T, NX, ROWS, NT_ROW, RO_KXINVCT, false>, g, NT_ROW, sm, st, u, tw);
-      case RO_STORE3: return launch_pass<T>(k_row_out<T, NX, ROWS, NT_ROW, RO_STORE3, true>, g, NT_ROW, sm, st, u, tw);
-      case RO_KXCT_DOT: return launch_pass<T>(k_row_out<T, NX, ROWS, NT_ROW, RO_KXCT_DOT, true>, g, NT_ROW, sm, st, u, tw);
-      default: return cudaErrorInvalidValue;
-    }
+  constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
+  const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
+  const dim3 g((Ny + G - 1) / G, maxcol, nunits);
+  switch (mode) {
+    case RO_KXCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT, true>, g, NT, sm, st, u, tw);
+    case RO_KXINVCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXINVCT, false>, g, NT, sm, st, u, tw);
+    case RO_STORE3: return launch_pass<T>(k_row_out2<T, NX, RO_STORE3, true>, g, NT, sm, st, u, tw);
+    case RO_KXCT_DOT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT_DOT, true>, g, NT, sm, st, u, tw);
+    default: return cudaErrorInvalidValue;
   }
 }
 
@@ -197,46 +165,34 @@ enum ColMode : int { CM_M = 0, CM_P = 1, CM_E = 2, CM_FWD = 3, CM_EPSINV = 4, CM
 template <typename T, int NY>
 static cudaError_t col_ny(int mode, const OpUnit<T>* u, int nunits, int Nx, int maxcol,
                           const cplx<T>* tw, cudaStream_t st, int tv = 1) {
-  if constexpr (plan2_a(NY) != 0 && sizeof(T) == 4) {
-    if (mode == CM_M && tv == 5)
+  if constexpr (sizeof(T) == 4) {
+    // (lines above 256 points: one register budget for both component-parallel variants, and variant 5
+    // is the default tile)
+    if (mode == CM_M && tv == 5 && NY <= 256)
       return col_b4<NY, CS_FWD, PW_EPS, CS_INV>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Nx, maxcol,
                                                 reinterpret_cast<const float2*>(tw), st);
     if (mode == CM_M && (tv == 3 || tv == 4)) {
       const auto* uf = reinterpret_cast<const OpUnit<float>*>(u);
       const auto* tf = reinterpret_cast<const float2*>(tw);
-      return tv == 3 ? col_sp<NY, CS_FWD, PW_EPS, CS_INV, 3>(uf, nunits, Nx, maxcol, tf, st)
-                     : col_sp<NY, CS_FWD, PW_EPS, CS_INV, 2>(uf, nunits, Nx, maxcol, tf, st);
+      constexpr int B3 = NY > 256 ? 1 : 3, B2 = NY > 256 ? 1 : 2;
+      return tv == 3 ? col_sp<NY, CS_FWD, PW_EPS, CS_INV, B3>(uf, nunits, Nx, maxcol, tf, st)
+                     : col_sp<NY, CS_FWD, PW_EPS, CS_INV, B2>(uf, nunits, Nx, maxcol, tf, st);
     }
-    if (mode == CM_M && tv != 1)
+    if (mode == CM_M && (tv == 0 || tv == 2))
       return tv == 0 ? col_tx<T, NY, col_tx_variant<NY>(0), CS_FWD, PW_EPS, CS_INV>(u, nunits, Nx, maxcol, tw, st)
                      : col_tx<T, NY, col_tx_variant<NY>(2), CS_FWD, PW_EPS, CS_INV>(u, nunits, Nx, maxcol, tw, st);
   }
-  if constexpr (plan2_a(NY) != 0) {  // two-level register FFT
-    constexpr int TX = l2_tx<T>(NY), NT = l2_col_threads<T>(NY);
-    const size_t sm = (size_t)3 * TX * l2_col_lstr<cplx<T>, NY, TX>() * sizeof(cplx<T>);
-    const dim3 g((Nx + TX - 1) / TX, maxcol, nunits);
-    switch (mode) {
-      case CM_M: return launch_pass<T>(k_col2<T, NY, CS_FWD, PW_EPS, CS_INV>, g, NT, sm, st, u, tw);
-      case CM_P: return launch_pass<T>(k_col2<T, NY, CS_INV, PW_EAVE, CS_FWD>, g, NT, sm, st, u, tw);
-      case CM_E: return launch_pass<T>(k_col2<T, NY, CS_FWD, PW_EPS, CS_NONE>, g, NT, sm, st, u, tw);
-      case CM_FWD: return launch_pass<T>(k_col2<T, NY, CS_FWD, PW_NONE, CS_NONE>, g, NT, sm, st, u, tw);
-      case CM_EPSINV: return launch_pass<T>(k_col2<T, NY, CS_NONE, PW_EPS, CS_INV>, g, NT, sm, st, u, tw);
-      case CM_BWD: return launch_pass<T>(k_col2<T, NY, CS_INV, PW_NONE, CS_NONE>, g, NT, sm, st, u, tw);
-      default: return cudaErrorInvalidValue;
-    }
-  } else {
-    constexpr int TX = tx_for<T>(NY);
-    const size_t sm = (NY + 3 * TX * (NY + 1)) * sizeof(cplx<T>);
-    const dim3 g((Nx + TX - 1) / TX, maxcol, nunits);
-    switch (mode) {
-      case CM_M: return launch_pass<T>(k_col<T, NY, TX, NT_COL, CS_FWD, PW_EPS, CS_INV>, g, NT_COL, sm, st, u, tw);
-      case CM_P: return launch_pass<T>(k_col<T, NY, TX, NT_COL, CS_INV, PW_EAVE, CS_FWD>, g, NT_COL, sm, st, u, tw);
-      case CM_E: return launch_pass<T>(k_col<T, NY, TX, NT_COL, CS_FWD, PW_EPS, CS_NONE>, g, NT_COL, sm, st, u, tw);
-      case CM_FWD: return launch_pass<T>(k_col<T, NY, TX, NT_COL, CS_FWD, PW_NONE, CS_NONE>, g, NT_COL, sm, st, u, tw);
-      case CM_EPSINV: return launch_pass<T>(k_col<T, NY, TX, NT_COL, CS_NONE, PW_EPS, CS_INV>, g, NT_COL, sm, st, u, tw);
-      case CM_BWD: return launch_pass<T>(k_col<T, NY, TX, NT_COL, CS_INV, PW_NONE, CS_NONE>, g, NT_COL, sm, st, u, tw);
-      default: return cudaErrorInvalidValue;
-    }
+  constexpr int TX = l2_tx<T>(NY), NT = l2_col_threads<T>(NY);
+  const size_t sm = (size_t)3 * TX * l2_col_lstr<cplx<T>, NY, TX>() * sizeof(cplx<T>);
+  const dim3 g((Nx + TX - 1) / TX, maxcol, nunits);
+  switch (mode) {
+    case CM_M: return launch_pass<T>(k_col2<T, NY, CS_FWD, PW_EPS, CS_INV>, g, NT, sm, st, u, tw);
+    case CM_P: return launch_pass<T>(k_col2<T, NY, CS_INV, PW_EAVE, CS_FWD>, g, NT, sm, st, u, tw);
+    case CM_E: return launch_pass<T>(k_col2<T, NY, CS_FWD, PW_EPS, CS_NONE>, g, NT, sm, st, u, tw);
+    case CM_FWD: return launch_pass<T>(k_col2<T, NY, CS_FWD, PW_NONE, CS_NONE>, g, NT, sm, st, u, tw);
+    case CM_EPSINV: return launch_pass<T>(k_col2<T, NY, CS_NONE, PW_EPS, CS_INV>, g, NT, sm, st, u, tw);
+    case CM_BWD: return launch_pass<T>(k_col2<T, NY, CS_INV, PW_NONE, CS_NONE>, g, NT, sm, st, u, tw);
+    default: return cudaErrorInvalidValue;
   }
 }
 

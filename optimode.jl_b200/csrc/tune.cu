@@ -3,10 +3,11 @@
 // the row-tile × column-tile × wave-size variants and the one-kernel cluster apply of an M̂ application on
 // device-resident data and keeps the fastest.  Choices live in a process-wide table keyed by
 // the device name and grid, persisted as text lines
-// "<device>|<Nx>|<Ny>|<row>|<col>|<seconds>|<wave>" in a cache file (OMB_TUNE_CACHE, else
+// "<device>|<Nx>|<Ny>|<row>|<col>|<seconds>|<wave>[|two-level]" in a cache file (OMB_TUNE_CACHE, else
 // $XDG_CACHE_HOME/omb200/tiles.txt, else ~/.cache/omb200/tiles.txt).
 #include <sys/stat.h>
 
+#include <algorithm>
 #include <cerrno>
 #include <cmath>
 #include <cstdio>
@@ -33,6 +34,9 @@ struct TuneEntry {
   int row = 1, col = 1;
   double seconds = 0;
   int wave = 0;
+  // read from a cache line written when lines above 256 points had one kernel whatever the variant: the
+  // choice is noise, so the grid runs with the defaults and counts as not tuned
+  bool stale = false;
 };
 using TuneKey = std::tuple<std::string, int, int>;
 std::mutex g_tune_mu;
@@ -49,21 +53,26 @@ std::string default_cache_path() {
   return base + "/omb200/tiles.txt";
 }
 
+// Grids with a line above 256 points carry an eighth field, naming the two-level passes they were
+// tuned on.
+const char* const LONG_LINES = "two-level";
+bool long_lines(int nx, int ny) { return std::max(nx, ny) > 256; }
+
 bool parse_line(const std::string& line, TuneKey& k, TuneEntry& e) {
   std::vector<std::string> f;
   std::stringstream ss(line);
   std::string item;
   while (std::getline(ss, item, '|')) f.push_back(item);
-  if ((f.size() != 6 && f.size() != 7) || f[0].empty()) return false;
+  if (f.size() < 6 || f.size() > 8 || f[0].empty() || (f.size() == 8 && f[7] != LONG_LINES)) return false;
   try {
     const int nx = std::stoi(f[1]), ny = std::stoi(f[2]), r = std::stoi(f[3]), c = std::stoi(f[4]);
     const double s = std::stod(f[5]);
-    const int w = f.size() == 7 ? std::stoi(f[6]) : 0;
+    const int w = f.size() >= 7 ? std::stoi(f[6]) : 0;
     if (nx <= 0 || ny <= 0 || r < 0 || r >= ROW_VARIANTS || c < 0 || c >= COL_VARIANTS || w < 0 ||
         w >= WAVE_VARIANTS || !(s >= 0))
       return false;
     k = TuneKey{f[0], nx, ny};
-    e = TuneEntry{r, c, s, w};
+    e = TuneEntry{r, c, s, w, long_lines(nx, ny) && f.size() < 8};
     return true;
   } catch (...) {
     return false;
@@ -94,7 +103,9 @@ int save_locked(const std::string& path) {
     if (!out) return fail(OMB_ERR_INVALID_ARG, "cannot write the tuning cache " + tmp);
     for (const auto& kv : g_tune)
       out << std::get<0>(kv.first) << '|' << std::get<1>(kv.first) << '|' << std::get<2>(kv.first) << '|'
-          << kv.second.row << '|' << kv.second.col << '|' << kv.second.seconds << '|' << kv.second.wave << '\n';
+          << kv.second.row << '|' << kv.second.col << '|' << kv.second.seconds << '|' << kv.second.wave
+          << (long_lines(std::get<1>(kv.first), std::get<2>(kv.first)) && !kv.second.stale ? std::string("|") + LONG_LINES : "")
+          << '\n';
   }
   if (std::rename(tmp.c_str(), path.c_str()) != 0) return fail(OMB_ERR_INVALID_ARG, "cannot replace " + path);
   return OMB_OK;
@@ -139,14 +150,15 @@ TileChoice tiles_for(int Nx, int Ny) {
   ensure_loaded_locked();
   auto it = g_tune.find(TuneKey{current_device_name_locked(), Nx, Ny});
   TileChoice t;
-  if (it != g_tune.end()) { t.row = it->second.row; t.col = it->second.col; t.wave = it->second.wave; }
+  if (it != g_tune.end() && !it->second.stale) { t.row = it->second.row; t.col = it->second.col; t.wave = it->second.wave; }
   return t;
 }
 
 bool tune_known(int dev, int Nx, int Ny) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   ensure_loaded_locked();
-  return g_tune.count(TuneKey{device_name_locked(dev), Nx, Ny}) > 0;
+  const auto it = g_tune.find(TuneKey{device_name_locked(dev), Nx, Ny});
+  return it != g_tune.end() && !it->second.stale;
 }
 
 // Times the tile × wave variants (168 slots; each cluster apply once) of one FP32 M̂ application to `ncol` columns on `units`

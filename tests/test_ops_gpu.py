@@ -220,3 +220,23 @@ def test_tile_variants_agree_and_autotune_picks_one():
         for rc in (5, 6):
             assert (t[rc] >= 0).sum() == (1 if (Nx, Ny) == (256, 256) else 0)
         assert ops.tune_get(name, Nx, Ny) == (r, c, w)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("Nx,Ny", [(320, 12), (8, 320), (384, 20), (40, 384), (512, 24), (12, 512), (384, 320)])
+def test_long_lines(omb, prec, Nx, Ny):
+    """Lines above 256 points (20·16, 24·16 and 32·16 points) beside short ones of every kind of
+    remainder (rows that do not fill a CTA's row block, columns that do not fill its tile): M̂, P̂, HMₖH
+    and E, at the tolerances of the other operator tests."""
+    g = omb.Grid(6.0, 4.0, Nx, Ny)
+    ei = random_epsinv(Nx, Ny, seed=Nx + 3 * Ny)
+    k = 1.23
+    H = rand_block(2 * g.N, 2, seed=Ny)
+    H /= np.linalg.norm(H, axis=0)
+    op = O.Operator(k, ei, O.Grid(6.0, 4.0, Nx, Ny))
+    assert rel(omb.apply_M(k, ei, g, H, precision=prec), op.M_block(H)) < TOL[prec]
+    assert rel(omb.apply_P(k, ei, g, H, precision=prec), op.P_block(H)) < TOL[prec]
+    ref = np.array([op.HMkH(H[:, j]) for j in range(2)])
+    scale = np.abs(op.HMkH(H[:, 0])) + k  # HMₖH of a random vector nearly cancels; compare on the operator's scale
+    assert np.max(np.abs(omb.HMkH(k, ei, g, H, precision=prec) - ref)) < TOL[prec] * scale * 40
+    assert rel(omb.E_field(k, ei, g, H[:, 0], precision=prec), O.E_field(k, H[:, 0], ei, O.Grid(6.0, 4.0, Nx, Ny))) < TOL[prec]
