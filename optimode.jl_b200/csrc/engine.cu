@@ -334,7 +334,16 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
     for (int L = 0; L < LANES; ++L) OMB_CU(d_exp[L].alloc((size_t)(maxNz + 1) * nt_, st));
 
   const char* step = "";
-  auto iteration = [&](int par, int L, cudaStream_t s) -> cudaError_t {
+  // The grid groups of a lane are independent between the lane's other kernels: in the graph they run on
+  // up to BRANCHES parallel branches.  A group's passes of a few tracks fill a fraction of the chip for
+  // 4–10 µs each, so one after the other they were the longest part of an uneven batch's iteration
+  // (ten cells of mixed sizes, one to three bands: 64.8 ms a solve in sequence, 54.1 branched).
+  constexpr int BRANCHES = 4;
+  struct Fork {
+    cudaStream_t st[BRANCHES] = {};
+    cudaEvent_t fork = nullptr, join[BRANCHES] = {};
+  };
+  auto iteration = [&](int par, int L, cudaStream_t s, const Fork* fk) -> cudaError_t {
     cudaError_t e = cudaSuccess;
     auto ok = [&](const char* name, cudaError_t r) { step = name; e = r; return r == cudaSuccess; };
     const int a = lane_lo[L], n = lane_hi[L] - lane_lo[L];
@@ -343,33 +352,47 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
     int* preu = preg + nt_ + 1;
     long long* wpreg = d_wpre_.p + (size_t)L * 2 * (nt_ + 1);
     long long* wpreu = wpreg + nt_ + 1;
-    auto op = [&](OpKind kind, const OpUnit<T>* u, int cnt, const Group& g, int maxcol) -> cudaError_t {
-      return g.Nz > 1 ? launch_op3d<T>(kind, u, cnt, g.Nx, g.Ny, g.Nz, maxcol, ctx_->tw, d_exp[L].p, s)
-                      : launch_op<T>(kind, u, cnt, g.Nx, g.Ny, maxcol, ctx_->tw, s);
+    auto op = [&](OpKind kind, const DevBuf<OpUnit<T>>& u, int off, int cnt, const Group& g, int maxcol,
+                  cudaStream_t gs) -> cudaError_t {
+      return g.Nz > 1 ? launch_op3d<T>(kind, u.p + off, cnt, g.Nx, g.Ny, g.Nz, maxcol, ctx_->tw,
+                                       d_exp[L].p + (size_t)(maxNz + 1) * off, gs)
+                      : launch_op<T>(kind, u.p + off, cnt, g.Nx, g.Ny, maxcol, ctx_->tw, gs);
     };
     // the lane's part of every grid group (its positions of the running wave)
-    auto for_groups = [&](auto&& f) -> bool {
-      for (size_t gi = 0; gi < groups_.size(); ++gi) {
-        const Group& g = groups_[gi];
-        const int lo = std::max(act_lo[gi], a), hi = std::min(act_hi[gi], a + n);
-        if (hi > lo && !f(g, lo, hi - lo)) return false;
+    auto for_groups = [&](const char* name, auto&& f) -> bool {
+      std::vector<int> mine;
+      for (size_t gi = 0; gi < groups_.size(); ++gi)
+        if (std::min(act_hi[gi], a + n) > std::max(act_lo[gi], a)) mine.push_back((int)gi);
+      const int nbr = fk ? std::min<int>(BRANCHES, (int)mine.size()) : 1;
+      if (nbr > 1 && !ok("branch fork", cudaEventRecord(fk->fork, s))) return false;
+      for (int q = 1; q < nbr; ++q)
+        if (!ok("branch fork", cudaStreamWaitEvent(fk->st[q], fk->fork, 0))) return false;
+      bool good = true;
+      for (size_t m = 0; m < mine.size() && good; ++m) {
+        const Group& g = groups_[mine[m]];
+        const int lo = std::max(act_lo[mine[m]], a), hi = std::min(act_hi[mine[m]], a + n), q = (int)m % nbr;
+        good = ok(name, f(g, lo, hi - lo, q == 0 ? s : fk->st[q]));
       }
-      return true;
+      for (int q = 1; q < nbr; ++q) {  // (joined after a failure too: a capture ends with every branch in it)
+        const cudaError_t j1 = cudaEventRecord(fk->join[q], fk->st[q]), j2 = cudaStreamWaitEvent(s, fk->join[q], 0);
+        if (good) good = ok("branch join", j1 != cudaSuccess ? j1 : j2);
+      }
+      return good;
     };
     if (!opt_.prec_diag &&
-        !for_groups([&](const Group& g, int off, int cnt) {
-          return ok("preconditioner pass", op(OP_P, d_uP[par].p + off, cnt, g, g.Mmax));
+        !for_groups("preconditioner pass", [&](const Group& g, int off, int cnt, cudaStream_t gs) {
+          return op(OP_P, d_uP[par], off, cnt, g, g.Mmax, gs);
         }))
       return e;
-    if (!for_groups([&](const Group& g, int off, int cnt) {
-          return ok("HMkH pass", op(OP_HMKH, d_uH[par].p + off, cnt, g, 1));
+    if (!for_groups("HMkH pass", [&](const Group& g, int off, int cnt, cudaStream_t gs) {
+          return op(OP_HMKH, d_uH[par], off, cnt, g, 1, gs);
         }))
       return e;
     k_newton<<<1, NEWTON_NT, 0, s>>>(d_state_ptrs_.p + a, d_hmkh_ptrs_.p + a, d_hmkh_nb_.p + a, d_n2_.p + a, n, rg,
                                      UpdCfg<T>::R, preg, preu, wpreg, wpreu, prm);
     if (!ok("k_newton", cudaGetLastError())) return e;
-    if (!for_groups([&](const Group& g, int off, int cnt) {
-          return ok("operator pass", op(OP_M, d_uA[par].p + off, cnt, g, 3 * g.Mmax));
+    if (!for_groups("operator pass", [&](const Group& g, int off, int cnt, cudaStream_t gs) {
+          return op(OP_M, d_uA[par], off, cnt, g, 3 * g.Mmax, gs);
         }))
       return e;
     k_gram<T><<<grid_g, GramCfg<T>::NT, sm_gram, s>>>(d_descs.p + a, preg, wpreg, n, par, nmax, rg, gstages,
@@ -387,7 +410,7 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
   // two eager iterations (they also size the kernels' shared memory), then the graph
   for (int par = 0; par < 2; ++par)
     for (int L = 0; L < nl; ++L) {
-      const cudaError_t e = iteration(par, L, st);
+      const cudaError_t e = iteration(par, L, st, nullptr);
       if (e != cudaSuccess) return cuda_fail(e, step);
     }
   cudaGraph_t graph = nullptr;
@@ -395,11 +418,18 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
   cudaStream_t lst[LANES] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[LANES] = {};
   lst[0] = st;
+  Fork forks[LANES];
+  const bool branched = groups_.size() > 1;
   auto release = [&]() {
     if (ev_fork) cudaEventDestroy(ev_fork);
-    for (int L = 1; L < LANES; ++L) {
-      if (ev_join[L]) cudaEventDestroy(ev_join[L]);
-      if (lst[L]) cudaStreamDestroy(lst[L]);
+    for (int L = 0; L < LANES; ++L) {
+      if (L > 0 && ev_join[L]) cudaEventDestroy(ev_join[L]);
+      if (L > 0 && lst[L]) cudaStreamDestroy(lst[L]);
+      if (forks[L].fork) cudaEventDestroy(forks[L].fork);
+      for (int q = 1; q < BRANCHES; ++q) {
+        if (forks[L].join[q]) cudaEventDestroy(forks[L].join[q]);
+        if (forks[L].st[q]) cudaStreamDestroy(forks[L].st[q]);
+      }
     }
   };
   {
@@ -407,6 +437,13 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
     for (int L = 1; L < nl && ce0 == cudaSuccess; ++L) {
       ce0 = cudaStreamCreateWithFlags(&lst[L], cudaStreamNonBlocking);
       if (ce0 == cudaSuccess) ce0 = cudaEventCreateWithFlags(&ev_join[L], cudaEventDisableTiming);
+    }
+    for (int L = 0; L < nl && branched && ce0 == cudaSuccess; ++L) {
+      ce0 = cudaEventCreateWithFlags(&forks[L].fork, cudaEventDisableTiming);
+      for (int q = 1; q < BRANCHES && ce0 == cudaSuccess; ++q) {
+        ce0 = cudaStreamCreateWithFlags(&forks[L].st[q], cudaStreamNonBlocking);
+        if (ce0 == cudaSuccess) ce0 = cudaEventCreateWithFlags(&forks[L].join[q], cudaEventDisableTiming);
+      }
     }
     if (ce0 != cudaSuccess) { release(); return cuda_fail(ce0, "lane streams"); }
   }
@@ -417,7 +454,7 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
     for (int L = 1; L < nl && ce == cudaSuccess; ++L) ce = cudaStreamWaitEvent(lst[L], ev_fork, 0);
   }
   for (int par = 0; par < 2 && ce == cudaSuccess; ++par)
-    for (int L = 0; L < nl && ce == cudaSuccess; ++L) ce = iteration(par, L, lst[L]);
+    for (int L = 0; L < nl && ce == cudaSuccess; ++L) ce = iteration(par, L, lst[L], branched ? &forks[L] : nullptr);
   for (int L = 1; L < nl; ++L) {
     const cudaError_t j1 = cudaEventRecord(ev_join[L], lst[L]);
     const cudaError_t j2 = cudaStreamWaitEvent(st, ev_join[L], 0);
