@@ -7,12 +7,12 @@
 // synchronisation of cudaMalloc/cudaFree.  This entry point takes every input and output as
 // caller-owned device memory and allocates nothing itself: the intermediate 3-component
 // field of the three FFT passes lives in a file-scope static device array of fixed size,
-// and so do the small per-call parameter block and the twiddle tables.
+// and so do the twiddle tables.
 //
 // Limits and rules:
 //  * Nx·Ny·ncol ≤ OMB_NOALLOC_MAX_PIXEL_COLUMNS (262144: e.g. 256×256 with 4 columns or
 //    512×512 with 1); larger requests are rejected with OMB_ERR_INVALID_ARG.
-//  * The array (6 MiB + 256 B) is held by every GPU that loads the library until exit.
+//  * The array (6 MiB) is held by every GPU that loads the library until exit.
 //  * All calls share it, so calls that overlap on the GPU (different streams, or
 //    different host threads) race; serialise them on one stream.
 //  * The first call in a CUDA context does a one-time set-up with that context current
@@ -20,10 +20,8 @@
 //    twiddle tables with a blocking copy); make that first call before any stream capture
 //    (a first call on a capturing stream is refused with OMB_ERR_INVALID_ARG).  The set-up
 //    is keyed on the context, so a new primary context after cudaDeviceReset repeats it.
-//  * Each call writes its parameter block (k and the pass descriptor) into the array with a
-//    one-thread kernel that receives them by value, on the caller's stream, ahead of the
-//    three passes; the field needs no clearing (the first pass writes every element the
-//    later passes read).
+//  * The pass descriptor travels as a kernel argument; the field needs no clearing (the first pass
+//    writes every element the later passes read).
 //  * The passes are the two-level register-FFT passes of omb_apply.  ε⁻¹ is read in the
 //    reference's (3, 3, Nx, Ny) layout.
 #include <cuda.h>
@@ -37,11 +35,10 @@
 namespace omb {
 
 constexpr long long NOALLOC_MAX_PIXEL_COLUMNS = 262144;
-constexpr size_t NOALLOC_PARAM_BYTES = 256;
 constexpr size_t NOALLOC_FIELD_BYTES = 3 * (size_t)NOALLOC_MAX_PIXEL_COLUMNS * sizeof(float2);
 
-// scratch: [0, 256) parameter block (k, then the pass descriptor), then the 3·N·ncol field
-static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_PARAM_BYTES + NOALLOC_FIELD_BYTES];
+// scratch: the 3·N·ncol field
+static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_FIELD_BYTES];
 
 #define OMB_NOALLOC_LENS(X) X(8) X(12) X(16) X(20) X(24) X(32) X(40) X(48) X(64) X(80) X(96) \
   X(128) X(160) X(192) X(256) X(320) X(384) X(512)
@@ -136,36 +133,57 @@ static int noalloc_setup(int dev, cudaStream_t st) {
   return OMB_OK;
 }
 
-// Writes the parameter block from kernel arguments, so no host memory is read later.
-__global__ void k_noalloc_params(OpUnit<float> u, double k, OpUnit<float>* ud, double* kd) {
-  *kd = k;
-  *ud = u;
+// The three passes in the component-parallel form (op_kernels_split.cuh) with the pass descriptor and k
+// passed by value: at this entry point's sizes a launch is at most one CTA per SM or so and its time is
+// one CTA's chain of latencies, which three times the threads shorten; and nothing has to be written
+// to the device ahead of it.  256×256 with 4 columns: 31.6 → 23.5 µs a call
+// (against a descriptor kernel and the one-thread-per-slot passes).
+struct NoallocUnit {
+  OpUnit<float> u;
+  double k;
+};
+__host__ __device__ constexpr int noalloc_tx(int NY) { return NY > 256 ? 4 : 8; }
+template <int NX>
+__global__ void __launch_bounds__(sp_row_threads(NX, l2_rows(NX)))
+    k_noalloc_row_in(const __grid_constant__ NoallocUnit P, const float2* __restrict__ tw) {
+  row_in_sp<float, NX, RI_KXTC, false, l2_rows(NX)>(P.u, P.k, tw);
+}
+template <int NY>
+__global__ void __launch_bounds__(sp_col_threads(NY, noalloc_tx(NY)))
+    k_noalloc_col(const __grid_constant__ NoallocUnit P, const float2* __restrict__ tw) {
+  col_sp<NY, CS_FWD, PW_EPS9, CS_INV, noalloc_tx(NY)>(P.u, blockIdx.y, tw);
+}
+template <int NX>
+__global__ void __launch_bounds__(sp_row_threads(NX, l2_rows(NX)))
+    k_noalloc_row_out(const __grid_constant__ NoallocUnit P, const float2* __restrict__ tw) {
+  row_out_sp<float, NX, RO_KXCT, true, l2_rows(NX)>(P.u, P.k, tw);
 }
 
 template <typename K> static cudaError_t noalloc_launch(K kern, dim3 g, int nt, size_t smem, cudaStream_t st,
-                                                         const OpUnit<float>* u, const float2* tw) {
+                                                         const NoallocUnit& P, const float2* tw) {
   if (smem > 32 * 1024) {
+    // (every call: the attribute belongs to the CUDA context, which may be a new one)
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<g, nt, smem, st>>>(u, tw);
+  kern<<<g, nt, smem, st>>>(P, tw);
   return cudaGetLastError();
 }
 
-template <int NX> static cudaError_t noalloc_rows(bool in, int Ny, int ncol, const OpUnit<float>* u,
+template <int NX> static cudaError_t noalloc_rows(bool in, int Ny, int ncol, const NoallocUnit& P,
                                                   const float2* tw, cudaStream_t st) {
-  constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
+  constexpr int G = l2_rows(NX), NT = sp_row_threads(NX, G);
   const size_t sm = (size_t)3 * G * l2_row_lstr<float2, NX>() * sizeof(float2);
   const dim3 g((Ny + G - 1) / G, ncol, 1);
-  return in ? noalloc_launch(k_row_in2<float, NX, RI_KXTC, false>, g, NT, sm, st, u, tw)
-            : noalloc_launch(k_row_out2<float, NX, RO_KXCT, true>, g, NT, sm, st, u, tw);
+  return in ? noalloc_launch(k_noalloc_row_in<NX>, g, NT, sm, st, P, tw)
+            : noalloc_launch(k_noalloc_row_out<NX>, g, NT, sm, st, P, tw);
 }
-template <int NY> static cudaError_t noalloc_col(int Nx, int ncol, const OpUnit<float>* u, const float2* tw,
+template <int NY> static cudaError_t noalloc_col(int Nx, int ncol, const NoallocUnit& P, const float2* tw,
                                                  cudaStream_t st) {
-  constexpr int TX = l2_tx<float>(NY), NT = l2_col_threads<float>(NY);
+  constexpr int TX = noalloc_tx(NY), NT = sp_col_threads(NY, TX);
   const size_t sm = (size_t)3 * TX * l2_col_lstr<float2, NY, TX>() * sizeof(float2);
   const dim3 g((Nx + TX - 1) / TX, ncol, 1);
-  return noalloc_launch(k_col2<float, NY, CS_FWD, PW_EPS9, CS_INV>, g, NT, sm, st, u, tw);
+  return noalloc_launch(k_noalloc_col<NY>, g, NT, sm, st, P, tw);
 }
 
 }  // namespace omb
@@ -192,38 +210,33 @@ extern "C" int omb_apply_M_noalloc(int32_t Nx, int32_t Ny, double Dx, double Dy,
   if (rc) return rc;
   const NoallocDevice& D = g_noalloc_dev[dev];
   const size_t N = (size_t)Nx * Ny;
-  // parameter block: k at offset 0, the pass descriptor at offset 64
-  double* kd = reinterpret_cast<double*>(D.scratch);
-  OpUnit<float>* ud = reinterpret_cast<OpUnit<float>*>(D.scratch + 64);
-  OpUnit<float> u{};
+  NoallocUnit P{};
+  P.k = k;
+  OpUnit<float>& u = P.u;
   u.in = static_cast<const float2*>(d_H_in);
   u.out = static_cast<float2*>(d_H_out);
-  u.scr = reinterpret_cast<float2*>(D.scratch + NOALLOC_PARAM_BYTES);
+  u.scr = reinterpret_cast<float2*>(D.scratch);
   u.e9 = d_epsinv;
-  u.k_dev = kd;
   u.in_cs = u.out_cs = (long long)(2 * N);
   u.scr_cs = (long long)(3 * N);
   u.Nx = Nx; u.Ny = Ny; u.ncol = ncol;
   u.part_stride = row_blocks(Nx, Ny);
   u.inv_dx = (float)(1.0 / Dx); u.inv_dy = (float)(1.0 / Dy);
-  static_assert(sizeof(OpUnit<float>) + 64 <= NOALLOC_PARAM_BYTES, "parameter block too small");
-  k_noalloc_params<<<1, 1, 0, st>>>(u, k, ud, kd);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "omb_apply_M_noalloc parameter block");
+  cudaError_t e = cudaSuccess;
   switch (Nx) {
-#define OMB_CASE(n) case n: e = noalloc_rows<n>(true, Ny, ncol, ud, D.tw + D.tw_off[n], st); break;
+#define OMB_CASE(n) case n: e = noalloc_rows<n>(true, Ny, ncol, P, D.tw + D.tw_off[n], st); break;
     OMB_NOALLOC_LENS(OMB_CASE)
 #undef OMB_CASE
   }
   if (e != cudaSuccess) return cuda_fail(e, "omb_apply_M_noalloc row pass");
   switch (Ny) {
-#define OMB_CASE(n) case n: e = noalloc_col<n>(Nx, ncol, ud, D.tw + D.tw_off[n], st); break;
+#define OMB_CASE(n) case n: e = noalloc_col<n>(Nx, ncol, P, D.tw + D.tw_off[n], st); break;
     OMB_NOALLOC_LENS(OMB_CASE)
 #undef OMB_CASE
   }
   if (e != cudaSuccess) return cuda_fail(e, "omb_apply_M_noalloc column pass");
   switch (Nx) {
-#define OMB_CASE(n) case n: e = noalloc_rows<n>(false, Ny, ncol, ud, D.tw + D.tw_off[n], st); break;
+#define OMB_CASE(n) case n: e = noalloc_rows<n>(false, Ny, ncol, P, D.tw + D.tw_off[n], st); break;
     OMB_NOALLOC_LENS(OMB_CASE)
 #undef OMB_CASE
   }

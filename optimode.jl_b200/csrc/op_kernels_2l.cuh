@@ -49,24 +49,25 @@ template <typename T> __host__ __device__ constexpr int l2_col_threads(int NY) {
   return l2_col_threads_tx(NY, l2_tx<T>(NY));
 }
 
-// Transverse basis for the pass kernels.  FP64 is basis_at itself; FP32 takes 1/|k+G| and
-// 1/|G| from the hardware reciprocal square root (≤ 2 ulp), which keeps the prologue and
-// epilogue at two MUFU operations per pixel instead of two square roots and two divisions.
-template <typename T> __device__ __forceinline__ Basis<T> basis_pass(T k, T gx, T gy) { return basis_at<T>(k, gx, gy); }
-template <> __device__ __forceinline__ Basis<float> basis_pass<float>(float k, float gx, float gy) {
-  Basis<float> b;
-  const float p2 = gx * gx + gy * gy, m2 = p2 + k * k;
-  const float im = rsqrtf(m2);
+// Transverse basis for the pass kernels (basis_at with 1/|k+G| and 1/|G| from reciprocal square
+// roots: ≤ 2 ulp; two such operations per pixel instead of two square roots and two divisions, which
+// in FP64 were more than half of a row pass's prologue).
+__device__ __forceinline__ float rsqrt_of(float x) { return rsqrtf(x); }
+__device__ __forceinline__ double rsqrt_of(double x) { return rsqrt(x); }
+template <typename T> __device__ __forceinline__ Basis<T> basis_pass(T k, T gx, T gy) {
+  Basis<T> b;
+  const T p2 = gx * gx + gy * gy, m2 = p2 + k * k;
+  const T im = rsqrt_of(m2);
   b.imag = im;
   b.mag = m2 * im;
-  if (p2 > 0.f) {
-    const float ip = rsqrtf(p2);
-    const float kim = k * ip * im;
+  if (p2 > T(0)) {
+    const T ip = rsqrt_of(p2);
+    const T kim = k * ip * im;
     b.nx = gy * ip; b.ny = -gx * ip;
     b.mx = -gx * kim; b.my = -gy * kim; b.mz = -p2 * ip * im;
   } else {
-    b.nx = 0.f; b.ny = 1.f;
-    b.mx = (k >= 0.f) ? 1.f : -1.f; b.my = 0.f; b.mz = 0.f;
+    b.nx = T(0); b.ny = T(1);
+    b.mx = (k >= T(0)) ? T(1) : T(-1); b.my = T(0); b.mz = T(0);
   }
   return b;
 }
@@ -232,13 +233,29 @@ __global__ void __launch_bounds__(l2_col_threads_tx(NY, TX), MINB)
   if constexpr (S1 != CS_NONE) {
     for (int q = threadIdx.x; q < TX * B; q += NT) {
       const int t = q % TX, n2 = q / TX, ix = ix0 + t;
+      // (lines of up to 16·16 points: the next component's loads are in flight while one is transformed)
+      constexpr bool AHEAD = A <= 16;
+      C v[A];
+      const C* Dc = D + (size_t)n2 * Nx + ix;
+#pragma unroll
+      for (int n1 = 0; n1 < A; ++n1) v[n1] = (ix < Nx) ? Dc[(size_t)(B * n1) * Nx] : mk<C>(0, 0);
 #pragma unroll 1
       for (int c = 0; c < 3; ++c) {
-        C v[A];
-        const C* Dc = D + c * N + (size_t)n2 * Nx + ix;
+        C nv[A];
+        Dc += N;
+        if constexpr (AHEAD) {
+          const bool more = c < 2 && ix < Nx;
 #pragma unroll
-        for (int n1 = 0; n1 < A; ++n1) v[n1] = (ix < Nx) ? Dc[(size_t)(B * n1) * Nx] : mk<C>(0, 0);
+          for (int n1 = 0; n1 < A; ++n1) nv[n1] = more ? Dc[(size_t)(B * n1) * Nx] : mk<C>(0, 0);
+        }
         l2_first<NY, S1 == CS_INV>(v, n2, blk + (c * TX + t) * LS, tw1);
+        if constexpr (!AHEAD) {
+          if (c < 2)
+#pragma unroll
+            for (int n1 = 0; n1 < A; ++n1) nv[n1] = (ix < Nx) ? Dc[(size_t)(B * n1) * Nx] : mk<C>(0, 0);
+        }
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) v[n1] = nv[n1];
       }
     }
     __syncthreads();

@@ -31,21 +31,18 @@ template <typename T> __host__ __device__ constexpr int sp_row_min_blocks(int nt
 // ------------------------------------------------------------------------------------
 // row_in.  Grid: (ceil(Ny/G), max columns, units); sp_row_threads(NX, G) threads.
 template <typename T, int NX, int MODE, bool INV, int G>
-__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G), NX))
-    k_row_in_sp(const OpUnit<T>* __restrict__ units, const cplx<T>* __restrict__ tw_g) {
+__device__ __forceinline__ void row_in_sp(const OpUnit<T>& U, double kd, const cplx<T>* __restrict__ tw_g) {
   using C = cplx<T>;
   constexpr int A = plan2_a(NX), B = NX / A, NT = sp_row_threads(NX, G);
   constexpr int LS = l2_row_lstr<C, NX>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* blk = reinterpret_cast<C*>(smem_raw);  // [3][G][LS]
-  const OpUnit<T>& U = units[blockIdx.z];
   const int col = blockIdx.y;
-  if (col >= unit_ncol(U)) return;
   const int Ny = U.Ny;
   const int row0 = blockIdx.x * G;
   if (row0 >= Ny) return;
   const size_t N = U.comp_stride ? (size_t)U.comp_stride : (size_t)NX * Ny;
-  const T k = (T)(*U.k_dev - U.kz_shift);
+  const T k = (T)(kd - U.kz_shift);
   const C* __restrict__ H = U.in + (size_t)(col + unit_col0(U)) * U.in_cs;
   // prologue, one thread per pixel (x fastest: coalesced loads of H), into the step-1 layout
   // x[B·n1 + n2] → block position n1·(B+1) + n2
@@ -82,23 +79,24 @@ __global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp
     for (int k2 = 0; k2 < B; ++k2) Dc[A * k2] = w[k2];
   }
 }
+template <typename T, int NX, int MODE, bool INV, int G>
+__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G), NX))
+    k_row_in_sp(const OpUnit<T>* __restrict__ units, const cplx<T>* __restrict__ tw_g) {
+  const OpUnit<T>& U = units[blockIdx.z];
+  if ((int)blockIdx.y < unit_ncol(U)) row_in_sp<T, NX, MODE, INV, G>(U, *U.k_dev, tw_g);
+}
 
 // ------------------------------------------------------------------------------------
 // col.  Grid: (ceil(Nx/TX), max columns, units); sp_col_threads(NY, TX) threads.
 // (MINB: CTAs per SM the register budget is set for; 3 leaves ≈56 registers a thread, 2 ≈85)
-template <int NY, int S1, int PW, int S2, int TX, int MINB = sp_min_blocks(sp_col_threads(NY, TX))>
-__global__ void __launch_bounds__(sp_col_threads(NY, TX), MINB)
-    k_col_sp(const OpUnit<float>* __restrict__ units, const float2* __restrict__ tw_g) {
+template <int NY, int S1, int PW, int S2, int TX>
+__device__ __forceinline__ void col_sp(const OpUnit<float>& U, int col, const float2* __restrict__ tw_g) {
   using T = float;
   using C = cplx<float>;
   constexpr int A = plan2_a(NY), B = NY / A, NT = sp_col_threads(NY, TX);
   constexpr int LS = l2_col_lstr<C, NY, TX>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* blk = reinterpret_cast<C*>(smem_raw);  // [3][TX][LS]
-  // vectors in the reverse of the row passes' order (the tiles row_in wrote last are in L2)
-  const OpUnit<T>& U = units[gridDim.z - 1 - blockIdx.z];
-  const int col = gridDim.y - 1 - blockIdx.y;
-  if (col >= unit_ncol(U)) return;
   const int Nx = U.Nx;
   const int ix0 = blockIdx.x * TX;
   if (ix0 >= Nx) return;
@@ -181,21 +179,26 @@ __global__ void __launch_bounds__(sp_col_threads(NY, TX), MINB)
     }
   }
 }
+template <int NY, int S1, int PW, int S2, int TX, int MINB = sp_min_blocks(sp_col_threads(NY, TX))>
+__global__ void __launch_bounds__(sp_col_threads(NY, TX), MINB)
+    k_col_sp(const OpUnit<float>* __restrict__ units, const float2* __restrict__ tw_g) {
+  // vectors in the reverse of the row passes' order (the tiles row_in wrote last are in L2)
+  const OpUnit<float>& U = units[gridDim.z - 1 - blockIdx.z];
+  const int col = gridDim.y - 1 - blockIdx.y;
+  if (col < unit_ncol(U)) col_sp<NY, S1, PW, S2, TX>(U, col, tw_g);
+}
 
 // ------------------------------------------------------------------------------------
 // row_out.  Grid: (ceil(Ny/G), max columns, units); sp_row_threads(NX, G) threads.
 template <typename T, int NX, int MODE, bool INV, int G>
-__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G), NX))
-    k_row_out_sp(const OpUnit<T>* __restrict__ units, const cplx<T>* __restrict__ tw_g) {
+__device__ __forceinline__ void row_out_sp(const OpUnit<T>& U, double kd, const cplx<T>* __restrict__ tw_g) {
   using C = cplx<T>;
   constexpr int A = plan2_a(NX), B = NX / A, NT = sp_row_threads(NX, G);
   constexpr int LS = l2_row_lstr<C, NX>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* blk = reinterpret_cast<C*>(smem_raw);  // [3][G][LS]
   __shared__ double red[2][NT / 32 + 1];
-  const OpUnit<T>& U = units[blockIdx.z];
   const int col = blockIdx.y;
-  if (col >= unit_ncol(U)) return;
   const int Ny = U.Ny;
   const int row0 = blockIdx.x * G;
   if (row0 >= Ny) return;
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp
     for (int m1 = 0; m1 < A; ++m1) line[m1 * (B + 1) + m2] = v[m1];
   }
   __syncthreads();
-  const T k = (T)(*U.k_dev - U.kz_shift);
+  const T k = (T)(kd - U.kz_shift);
   const T sN = T(1) / T(N);
   const int c0 = unit_col0(U);
   C* __restrict__ O = U.out + (size_t)(col + c0) * U.out_cs;
@@ -274,6 +277,12 @@ __global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp
       P[0] = sr; P[1] = si;
     }
   }
+}
+template <typename T, int NX, int MODE, bool INV, int G>
+__global__ void __launch_bounds__(sp_row_threads(NX, G), sp_row_min_blocks<T>(sp_row_threads(NX, G), NX))
+    k_row_out_sp(const OpUnit<T>* __restrict__ units, const cplx<T>* __restrict__ tw_g) {
+  const OpUnit<T>& U = units[blockIdx.z];
+  if ((int)blockIdx.y < unit_ncol(U)) row_out_sp<T, NX, MODE, INV, G>(U, *U.k_dev, tw_g);
 }
 
 }  // namespace omb

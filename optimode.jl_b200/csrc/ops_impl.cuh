@@ -77,23 +77,26 @@ static cudaError_t col_tx(const OpUnit<T>* u, int nunits, int Nx, int maxcol, co
 }
 
 template <int NX, int MODE, bool INV, typename T = float>
-static cudaError_t row_in_sp(const OpUnit<T>* u, int nunits, int Ny, int maxcol, const cplx<T>* tw, cudaStream_t st) {
+static cudaError_t launch_row_in_sp(const OpUnit<T>* u, int nunits, int Ny, int maxcol, const cplx<T>* tw, cudaStream_t st) {
   constexpr int G = l2_rows(NX), NT = sp_row_threads(NX, G);
   const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
   const dim3 g((Ny + G - 1) / G, maxcol, nunits);
   return launch_pass<T>(k_row_in_sp<T, NX, MODE, INV, G>, g, NT, sm, st, u, tw);
 }
 template <int NX, int MODE, bool INV, typename T = float>
-static cudaError_t row_out_sp(const OpUnit<T>* u, int nunits, int Ny, int maxcol, const cplx<T>* tw, cudaStream_t st) {
+static cudaError_t launch_row_out_sp(const OpUnit<T>* u, int nunits, int Ny, int maxcol, const cplx<T>* tw, cudaStream_t st) {
   constexpr int G = l2_rows(NX), NT = sp_row_threads(NX, G);
   const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
   const dim3 g((Ny + G - 1) / G, maxcol, nunits);
   return launch_pass<T>(k_row_out_sp<T, NX, MODE, INV, G>, g, NT, sm, st, u, tw);
 }
-// FP64 M̂ row passes in the component-parallel form (one thread per line slot and component)
-constexpr bool FP64_ROW_SPLIT = true;
+// Whether every mode of a row pass takes the component-parallel form (one thread per line slot and
+// component): FP64, and FP32 lines above 256 points, where a thread holding three components of 20–32
+// points spills.  (The MPB preconditioner's FP64 row passes on 192×128 with two
+// columns: 16.3 and 11.8 µs with one thread per slot, 8.6 and 7.4 so.)
+template <typename T> __host__ __device__ constexpr bool row_split(int NX) { return sizeof(T) == 8 || NX > 256; }
 template <int NY, int S1, int PW, int S2, int MINB>
-static cudaError_t col_sp(const OpUnit<float>* u, int nunits, int Nx, int maxcol, const float2* tw, cudaStream_t st) {
+static cudaError_t launch_col_sp(const OpUnit<float>* u, int nunits, int Nx, int maxcol, const float2* tw, cudaStream_t st) {
   constexpr int TX = l2_tx<float>(NY), NT = sp_col_threads(NY, TX);
   const size_t sm = (size_t)3 * TX * l2_col_lstr<float2, NY, TX>() * sizeof(float2);
   const dim3 g((Nx + TX - 1) / TX, maxcol, nunits);
@@ -105,25 +108,33 @@ static cudaError_t row_in_nx(int mode, const OpUnit<T>* u, int nunits, int Ny, i
                              const cplx<T>* tw, cudaStream_t st, int gv = 1) {
   if constexpr (sizeof(T) == 4) {
     if (mode == RI_KXTC && (gv == 3 || gv == 4))
-      return row_in_sp<NX, RI_KXTC, false>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Ny, maxcol,
+      return launch_row_in_sp<NX, RI_KXTC, false>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Ny, maxcol,
                                            reinterpret_cast<const float2*>(tw), st);
     if (mode == RI_KXTC && gv != 1)
       return gv == 0 ? row_in_g<T, NX, row_g_variant<NX>(0), RI_KXTC, false>(u, nunits, Ny, maxcol, tw, st)
                      : row_in_g<T, NX, row_g_variant<NX>(2), RI_KXTC, false>(u, nunits, Ny, maxcol, tw, st);
   }
-  if constexpr (sizeof(T) == 8) {
-    if (FP64_ROW_SPLIT && mode == RI_KXTC) return row_in_sp<NX, RI_KXTC, false, T>(u, nunits, Ny, maxcol, tw, st);
-  }
-  constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
-  const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
-  const dim3 g((Ny + G - 1) / G, maxcol, nunits);
-  switch (mode) {
-    case RI_KXTC: return launch_pass<T>(k_row_in2<T, NX, RI_KXTC, false>, g, NT, sm, st, u, tw);
-    case RI_KXINV: return launch_pass<T>(k_row_in2<T, NX, RI_KXINV, true>, g, NT, sm, st, u, tw);
-    case RI_ZXTC: return launch_pass<T>(k_row_in2<T, NX, RI_ZXTC, false>, g, NT, sm, st, u, tw);
-    case RI_HCART: return launch_pass<T>(k_row_in2<T, NX, RI_HCART, false>, g, NT, sm, st, u, tw);
-    case RI_LOAD3: return launch_pass<T>(k_row_in2<T, NX, RI_LOAD3, true>, g, NT, sm, st, u, tw);
-    default: return cudaErrorInvalidValue;
+  if constexpr (row_split<T>(NX)) {
+    switch (mode) {
+      case RI_KXTC: return launch_row_in_sp<NX, RI_KXTC, false, T>(u, nunits, Ny, maxcol, tw, st);
+      case RI_KXINV: return launch_row_in_sp<NX, RI_KXINV, true, T>(u, nunits, Ny, maxcol, tw, st);
+      case RI_ZXTC: return launch_row_in_sp<NX, RI_ZXTC, false, T>(u, nunits, Ny, maxcol, tw, st);
+      case RI_HCART: return launch_row_in_sp<NX, RI_HCART, false, T>(u, nunits, Ny, maxcol, tw, st);
+      case RI_LOAD3: return launch_row_in_sp<NX, RI_LOAD3, true, T>(u, nunits, Ny, maxcol, tw, st);
+      default: return cudaErrorInvalidValue;
+    }
+  } else {
+    constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
+    const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
+    const dim3 g((Ny + G - 1) / G, maxcol, nunits);
+    switch (mode) {
+      case RI_KXTC: return launch_pass<T>(k_row_in2<T, NX, RI_KXTC, false>, g, NT, sm, st, u, tw);
+      case RI_KXINV: return launch_pass<T>(k_row_in2<T, NX, RI_KXINV, true>, g, NT, sm, st, u, tw);
+      case RI_ZXTC: return launch_pass<T>(k_row_in2<T, NX, RI_ZXTC, false>, g, NT, sm, st, u, tw);
+      case RI_HCART: return launch_pass<T>(k_row_in2<T, NX, RI_HCART, false>, g, NT, sm, st, u, tw);
+      case RI_LOAD3: return launch_pass<T>(k_row_in2<T, NX, RI_LOAD3, true>, g, NT, sm, st, u, tw);
+      default: return cudaErrorInvalidValue;
+    }
   }
 }
 
@@ -135,27 +146,34 @@ static cudaError_t row_out_nx(int mode, const OpUnit<T>* u, int nunits, int Ny, 
     if (mode == RO_KXCT && gv == 3)
       return row_out_nx<T, NX>(mode, u, nunits, Ny, maxcol, tw, st, 1);
     if (mode == RO_KXCT && gv == 4)
-      return row_out_sp<NX, RO_KXCT, true>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Ny, maxcol,
+      return launch_row_out_sp<NX, RO_KXCT, true>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Ny, maxcol,
                                            reinterpret_cast<const float2*>(tw), st);
     if (mode == RO_KXCT_DOT && gv == 4)
-      return row_out_sp<NX, RO_KXCT_DOT, true>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Ny, maxcol,
+      return launch_row_out_sp<NX, RO_KXCT_DOT, true>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Ny, maxcol,
                                                reinterpret_cast<const float2*>(tw), st);
     if (mode == RO_KXCT && gv != 1)
       return gv == 0 ? row_out_g<T, NX, row_g_variant<NX>(0), RO_KXCT, true>(u, nunits, Ny, maxcol, tw, st)
                      : row_out_g<T, NX, row_g_variant<NX>(2), RO_KXCT, true>(u, nunits, Ny, maxcol, tw, st);
   }
-  if constexpr (sizeof(T) == 8) {
-    if (FP64_ROW_SPLIT && mode == RO_KXCT) return row_out_sp<NX, RO_KXCT, true, T>(u, nunits, Ny, maxcol, tw, st);
-  }
-  constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
-  const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
-  const dim3 g((Ny + G - 1) / G, maxcol, nunits);
-  switch (mode) {
-    case RO_KXCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT, true>, g, NT, sm, st, u, tw);
-    case RO_KXINVCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXINVCT, false>, g, NT, sm, st, u, tw);
-    case RO_STORE3: return launch_pass<T>(k_row_out2<T, NX, RO_STORE3, true>, g, NT, sm, st, u, tw);
-    case RO_KXCT_DOT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT_DOT, true>, g, NT, sm, st, u, tw);
-    default: return cudaErrorInvalidValue;
+  if constexpr (row_split<T>(NX)) {
+    switch (mode) {
+      case RO_KXCT: return launch_row_out_sp<NX, RO_KXCT, true, T>(u, nunits, Ny, maxcol, tw, st);
+      case RO_KXINVCT: return launch_row_out_sp<NX, RO_KXINVCT, false, T>(u, nunits, Ny, maxcol, tw, st);
+      case RO_STORE3: return launch_row_out_sp<NX, RO_STORE3, true, T>(u, nunits, Ny, maxcol, tw, st);
+      case RO_KXCT_DOT: return launch_row_out_sp<NX, RO_KXCT_DOT, true, T>(u, nunits, Ny, maxcol, tw, st);
+      default: return cudaErrorInvalidValue;
+    }
+  } else {
+    constexpr int G = l2_rows(NX), NT = l2_row_threads(NX);
+    const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
+    const dim3 g((Ny + G - 1) / G, maxcol, nunits);
+    switch (mode) {
+      case RO_KXCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT, true>, g, NT, sm, st, u, tw);
+      case RO_KXINVCT: return launch_pass<T>(k_row_out2<T, NX, RO_KXINVCT, false>, g, NT, sm, st, u, tw);
+      case RO_STORE3: return launch_pass<T>(k_row_out2<T, NX, RO_STORE3, true>, g, NT, sm, st, u, tw);
+      case RO_KXCT_DOT: return launch_pass<T>(k_row_out2<T, NX, RO_KXCT_DOT, true>, g, NT, sm, st, u, tw);
+      default: return cudaErrorInvalidValue;
+    }
   }
 }
 
@@ -175,8 +193,8 @@ static cudaError_t col_ny(int mode, const OpUnit<T>* u, int nunits, int Nx, int 
       const auto* uf = reinterpret_cast<const OpUnit<float>*>(u);
       const auto* tf = reinterpret_cast<const float2*>(tw);
       constexpr int B3 = NY > 256 ? 1 : 3, B2 = NY > 256 ? 1 : 2;
-      return tv == 3 ? col_sp<NY, CS_FWD, PW_EPS, CS_INV, B3>(uf, nunits, Nx, maxcol, tf, st)
-                     : col_sp<NY, CS_FWD, PW_EPS, CS_INV, B2>(uf, nunits, Nx, maxcol, tf, st);
+      return tv == 3 ? launch_col_sp<NY, CS_FWD, PW_EPS, CS_INV, B3>(uf, nunits, Nx, maxcol, tf, st)
+                     : launch_col_sp<NY, CS_FWD, PW_EPS, CS_INV, B2>(uf, nunits, Nx, maxcol, tf, st);
     }
     if (mode == CM_M && (tv == 0 || tv == 2))
       return tv == 0 ? col_tx<T, NY, col_tx_variant<NY>(0), CS_FWD, PW_EPS, CS_INV>(u, nunits, Nx, maxcol, tw, st)
