@@ -144,9 +144,9 @@ struct NoallocUnit {
 };
 __host__ __device__ constexpr int noalloc_tx(int NY) { return NY > 256 ? 4 : 8; }
 template <int NX>
-__global__ void __launch_bounds__(sp_row_threads(NX, l2_rows(NX)))
+__global__ void __launch_bounds__(sp_row_threads(NX, sp_rows(NX)), sp_row_min_blocks<float>(sp_row_threads(NX, sp_rows(NX)), NX))
     k_noalloc_row_in(const __grid_constant__ NoallocUnit P, const float2* __restrict__ tw) {
-  row_in_sp<float, NX, RI_KXTC, false, l2_rows(NX)>(P.u, P.k, tw);
+  row_in_sp<float, NX, RI_KXTC, false, sp_rows(NX)>(P.u, P.k, tw);
 }
 template <int NY>
 __global__ void __launch_bounds__(sp_col_threads(NY, noalloc_tx(NY)))
@@ -154,9 +154,9 @@ __global__ void __launch_bounds__(sp_col_threads(NY, noalloc_tx(NY)))
   col_sp<NY, CS_FWD, PW_EPS9, CS_INV, noalloc_tx(NY)>(P.u, blockIdx.y, tw);
 }
 template <int NX>
-__global__ void __launch_bounds__(sp_row_threads(NX, l2_rows(NX)))
+__global__ void __launch_bounds__(sp_row_threads(NX, sp_rows(NX)), sp_row_min_blocks<float>(sp_row_threads(NX, sp_rows(NX)), NX))
     k_noalloc_row_out(const __grid_constant__ NoallocUnit P, const float2* __restrict__ tw) {
-  row_out_sp<float, NX, RO_KXCT, true, l2_rows(NX)>(P.u, P.k, tw);
+  row_out_sp<float, NX, RO_KXCT, true, sp_rows(NX)>(P.u, P.k, tw);
 }
 
 template <typename K> static cudaError_t noalloc_launch(K kern, dim3 g, int nt, size_t smem, cudaStream_t st,
@@ -172,7 +172,7 @@ template <typename K> static cudaError_t noalloc_launch(K kern, dim3 g, int nt, 
 
 template <int NX> static cudaError_t noalloc_rows(bool in, int Ny, int ncol, const NoallocUnit& P,
                                                   const float2* tw, cudaStream_t st) {
-  constexpr int G = l2_rows(NX), NT = sp_row_threads(NX, G);
+  constexpr int G = sp_rows(NX), NT = sp_row_threads(NX, G);
   const size_t sm = (size_t)3 * G * l2_row_lstr<float2, NX>() * sizeof(float2);
   const dim3 g((Ny + G - 1) / G, ncol, 1);
   return in ? noalloc_launch(k_noalloc_row_in<NX>, g, NT, sm, st, P, tw)

@@ -20,12 +20,19 @@ namespace omb {
 
 __host__ __device__ constexpr int sp_row_threads(int NX, int G) { return (3 * G * plan2_max(NX) + 31) / 32 * 32; }
 __host__ __device__ constexpr int sp_col_threads(int NY, int TX) { return (3 * TX * plan2_max(NY) + 31) / 32 * 32; }
-// CTAs per SM the register budget is set for (the 52 KB FP32 block allows four; an FP64 row
-// block is twice as large and its A or B complex doubles need ≈80 registers)
+// CTAs per SM the column pass's register budget is set for
 __host__ __device__ constexpr int sp_min_blocks(int nt) { return nt <= 384 ? 3 : (nt <= 512 ? 2 : 1); }
-// (lines above 256 points hold up to 32 of a component: two FP32 CTAs, one FP64)
+// Rows per CTA of the row passes: a quarter of the one-thread-per-slot passes' (2 at 256 points), so
+// that more and smaller CTAs share an SM and one's barriers and loads overlap the others' arithmetic.
+// One M̂ application at 256², 8 → 2 rows: 4 columns of 64 cells in FP32 524 → 488 µs, of 32 cells in FP64
+// 662 → 622; 5 columns of one cell 27 → 24 and 47 → 41; one column at 128² 17.6 → 14.6 and 22.3 → 19.7.
+// (The dot-product epilogue keeps l2_rows: its partial sums are laid out per row block.)
+__host__ __device__ constexpr int sp_rows(int NX) { return l2_rows(NX) / 4 > 0 ? l2_rows(NX) / 4 : 1; }
+// Threads per SM the row passes' register budget is set for: 1152 in FP32 (56 registers a thread),
+// 768 in FP64 (85); lines above 256 points, up to 32 points of a component a thread, 768 and 384.
 template <typename T> __host__ __device__ constexpr int sp_row_min_blocks(int nt, int NX) {
-  return NX > 256 ? (sizeof(T) == 4 ? 2 : 1) : (sizeof(T) == 4 ? sp_min_blocks(nt) : (nt <= 512 ? 2 : 1));
+  const int budget = sizeof(T) == 4 ? (NX > 256 ? 768 : 1152) : (NX > 256 ? 384 : 768);
+  return budget / nt > 1 ? budget / nt : 1;
 }
 
 // ------------------------------------------------------------------------------------

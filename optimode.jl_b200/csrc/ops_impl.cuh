@@ -78,14 +78,14 @@ static cudaError_t col_tx(const OpUnit<T>* u, int nunits, int Nx, int maxcol, co
 
 template <int NX, int MODE, bool INV, typename T = float>
 static cudaError_t launch_row_in_sp(const OpUnit<T>* u, int nunits, int Ny, int maxcol, const cplx<T>* tw, cudaStream_t st) {
-  constexpr int G = l2_rows(NX), NT = sp_row_threads(NX, G);
+  constexpr int G = sp_rows(NX), NT = sp_row_threads(NX, G);
   const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
   const dim3 g((Ny + G - 1) / G, maxcol, nunits);
   return launch_pass<T>(k_row_in_sp<T, NX, MODE, INV, G>, g, NT, sm, st, u, tw);
 }
 template <int NX, int MODE, bool INV, typename T = float>
 static cudaError_t launch_row_out_sp(const OpUnit<T>* u, int nunits, int Ny, int maxcol, const cplx<T>* tw, cudaStream_t st) {
-  constexpr int G = l2_rows(NX), NT = sp_row_threads(NX, G);
+  constexpr int G = MODE == RO_KXCT_DOT ? l2_rows(NX) : sp_rows(NX), NT = sp_row_threads(NX, G);
   const size_t sm = (size_t)3 * G * l2_row_lstr<cplx<T>, NX>() * sizeof(cplx<T>);
   const dim3 g((Ny + G - 1) / G, maxcol, nunits);
   return launch_pass<T>(k_row_out_sp<T, NX, MODE, INV, G>, g, NT, sm, st, u, tw);
