@@ -158,8 +158,26 @@ struct TileWalk {
   __device__ __forceinline__ bool last_of_track() const { return i + 1 >= end || pre[t + 1] <= i + 1; }
 };
 
-// Relative cost of one tile of a track with n block columns of which M are X: the Gram's 4×4
-// items (each 16 complex products per row) plus its loads plus a fixed GRAM_TILE_FIXED, and
+// The prefixes in shared memory, when the lane has few enough tracks: TileWalk's searches are chains of
+// dependent reads, which from global memory (≈0.35 µs each) were a third of a small launch's time.
+// Every thread of the CTA calls it before a __syncthreads.
+constexpr int TRACKS_SH = 128;
+struct PrefixSh {
+  int pre[TRACKS_SH + 1];
+  long long wpre[TRACKS_SH + 1];
+};
+__device__ __forceinline__ void stage_prefixes(PrefixSh& sh, const int*& pre, const long long*& wpre, int ntracks) {
+  if (ntracks > TRACKS_SH) return;
+  for (int i = threadIdx.x; i <= ntracks; i += blockDim.x) {
+    sh.pre[i] = pre[i];
+    if (wpre) sh.wpre[i] = wpre[i];
+  }
+  pre = sh.pre;
+  if (wpre) wpre = sh.wpre;
+}
+
+// Relative cost of one tile of a track with n block columns of which M are X: the Gram's items (18
+// complex products per row, two to the unit) plus its loads plus a fixed GRAM_TILE_FIXED, and
 // GRAM_TRACK_COST once per track for the flush of its sums (each CTA that takes part in a
 // track adds its partial sums to the track's Gram); the update's n·M products per row of X,
 // AX, P, AP plus its 4M stores plus a fixed 16 per tile (pipeline round trips and bulk-copy
@@ -167,49 +185,54 @@ struct TileWalk {
 constexpr long long GRAM_TILE_FIXED = 48;
 constexpr long long GRAM_TRACK_COST = 390;
 __host__ __device__ __forceinline__ long long gram_tile_cost(int n) {
-  const int nb4 = (n + 3) / 4;
-  return 8LL * nb4 * (nb4 + 1) + n + GRAM_TILE_FIXED;
+  const int nb = (n + 2) / 3;
+  return 9LL * (nb * (nb + 1) / 2) + n + GRAM_TILE_FIXED;
 }
 __host__ __device__ __forceinline__ long long update_tile_cost(int n, int M) { return (long long)n * M + 4LL * M + 16; }
 
 // ---- Gram ---------------------------------------------------------------------------
-// G = ZᴴZ and S = ZᴴAZ (upper triangles).  The outputs are cut into 4×4 blocks (items);
-// items·SPLIT ≤ 512 consumer threads, each thread owns one item and every SPLIT-th row of
-// a tile (16 complex accumulators), and the SPLIT threads of an item are adjacent lanes,
-// so their partial sums meet in a shuffle reduction (FP64) before the atomics.
+// G = ZᴴZ and S = ZᴴAZ (upper triangles).  The outputs are cut into 3×3 blocks; an item is the block
+// (bi, bj) of both matrices, so that the three rows of Z it multiplies are read from shared memory once
+// for 18 products (9 reads).  Three divides the usual basis of 3M columns: against separate 4×4
+// blocks of G and S (8 reads for 16 products, and up to half of the products outside the triangle)
+// a row takes 24 % fewer products and reads over the tracks of a four-band solve (n = 6, 9, 12, 15):
+// with the prefixes in shared memory and the flush below, the sweep of twelve 256² instances 314 → 293 ms,
+// one 256² solve 56.7 → 53.3.  Each consumer thread owns one item and every split-th row of a tile (18 complex
+// accumulators), and the split threads of an item are adjacent lanes, so their partial sums meet in a
+// shuffle reduction (FP64) before the atomics.
+constexpr int GRAM_B = 3;                     // block side
+constexpr int GRAM_E = 2 * GRAM_B * GRAM_B;   // entries of an item
+__host__ __device__ constexpr int gram_nb(int n) { return (n + GRAM_B - 1) / GRAM_B; }
+__host__ __device__ constexpr int gram_items(int n) { return gram_nb(n) * (gram_nb(n) + 1) / 2; }
 template <typename T> struct GramCfg {
   static constexpr int NCW = 15;                                 // consumer warps
   static constexpr int NT = (NCW + 1) * 32;                      // + the producer warp (16 warps: 128 regs;
                                                                  // FP32 keeps its compensation terms in local memory)
   static constexpr int PAD = 16 / (int)sizeof(cplx<T>);          // column pad: 16 bytes
-  // Z columns at [0, n), AZ columns at [n4, n4 + n) with n4 = 4·⌈n/4⌉: the 4×4 blocks read
-  // up to column 2·n4 − 1, so a stage holds 2·4·⌈nmax/4⌉ columns of R + PAD elements
-  static __host__ __device__ constexpr int n4(int n) { return (n + 3) / 4 * 4; }
-  static __host__ __device__ constexpr size_t stage_elems(int nmax, int R) { return (size_t)2 * n4(nmax) * (R + PAD); }
+  // Z columns at [0, n), AZ columns at [nr, nr + n) with nr = 3·⌈n/3⌉: the blocks read
+  // up to column 2·nr − 1, so a stage holds 2·3·⌈nmax/3⌉ columns of R + PAD elements
+  static __host__ __device__ constexpr int nr(int n) { return GRAM_B * gram_nb(n); }
+  static __host__ __device__ constexpr size_t stage_elems(int nmax, int R) { return (size_t)2 * nr(nmax) * (R + PAD); }
   // rows per tile: the largest multiple of 64 (≤ 256 FP32, ≤ 128 FP64) whose stage fits in ≈95 KB
   static __host__ int rows(int nmax) {
     const int cap = sizeof(T) == 4 ? 256 : 128;
-    int R = (int)(95 * 1024 / (2 * n4(nmax) * sizeof(cplx<T>))) - PAD;
+    int R = (int)(95 * 1024 / (2 * nr(nmax) * sizeof(cplx<T>))) - PAD;
     R = R / 64 * 64;
     return R < 64 ? 64 : (R > cap ? cap : R);
   }
-  // FP64 reduction buffer after the ring: 16 entries per item
-  static __host__ __device__ constexpr int red_entries(int nmax) {
-    return 2 * ((nmax + 3) / 4) * ((nmax + 3) / 4 + 1) / 2 * 16;
-  }
+  // FP64 reduction buffer after the ring
+  static __host__ __device__ constexpr int red_entries(int nmax) { return GRAM_E * gram_items(nmax); }
 };
 
 // Named barrier over the first `count` threads of the CTA (the consumer warps).
 __device__ __forceinline__ void bar_sync_count(int id, int count) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory");
 }
-// Item q of a track with nb4 column blocks: matrix (0: G, 1: S) and block (bi ≤ bj).
-__device__ __forceinline__ void gram_item(int q, int nblk, int nb4, int& which, int& bi, int& bj) {
-  which = q / nblk;
-  int r = q - which * nblk;
+// Block (bi ≤ bj) of item q of a track with nb column blocks.
+__device__ __forceinline__ void gram_item(int q, int nb, int& bi, int& bj) {
   bi = 0;
-  while (r >= nb4 - bi) { r -= nb4 - bi; ++bi; }
-  bj = bi + r;
+  while (q >= nb - bi) { q -= nb - bi; ++bi; }
+  bj = bi + q;
 }
 
 // s + lo += x with the rounding error of the FP32 addition carried in lo (two-sum: Knuth,
@@ -222,20 +245,46 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& lo, float x) {
 }
 
 // (acc, lo) += t entry by entry with two-sum; t is cleared.
-__device__ __forceinline__ void gram_fold(float2 (&acc)[4][4], float2 (&lo)[4][4], float2 (&t)[4][4]) {
+__device__ __forceinline__ void gram_fold(float2 (&acc)[GRAM_E], float2 (&lo)[GRAM_E], float2 (&t)[GRAM_E]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int e = 0; e < GRAM_E; ++e) {
+    two_sum_acc(acc[e].x, lo[e].x, t[e].x);
+    two_sum_acc(acc[e].y, lo[e].y, t[e].y);
+    t[e] = make_float2(0.f, 0.f);
+  }
+}
+
+// Adds the sums of 12 values over the lanes of a warp to out[0..11].  Each step exchanges half of the
+// values with the lane 16, 8, 4, 2, 1 away, which sums the other half: 12 → 6 → 3 → 2 → 1 → 1 values a
+// lane (padded with zeros), 13 shuffles instead of 12·5, and the final adds of a warp fall on distinct
+// addresses.  (An item's 36 values go in three such groups: all at once is as many shuffles, but their
+// registers spill around the row loop and cost the sweep of twelve 256² instances 9 %.)
+constexpr int GRAM_SUM = 12;
+__device__ __forceinline__ void gram_warp_sum(double (&v)[GRAM_SUM], int lane, double* out) {
+  int at = 0;  // index of the lane's first value
+  auto halve = [&](auto from, int o) {
+    constexpr int F = decltype(from)::value, K = (F + 1) / 2;
+    const bool up = lane & o;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      two_sum_acc(acc[i][j].x, lo[i][j].x, t[i][j].x);
-      two_sum_acc(acc[i][j].y, lo[i][j].y, t[i][j].y);
-      t[i][j] = make_float2(0.f, 0.f);
+    for (int k = 0; k < K; ++k) {
+      const double hi = K + k < F ? v[K + k] : 0.0;
+      const double got = __shfl_xor_sync(0xffffffffu, up ? v[k] : hi, o);
+      v[k] = (up ? hi : v[k]) + got;
     }
+    at += up ? K : 0;
+  };
+  halve(std::integral_constant<int, 12>{}, 16);
+  halve(std::integral_constant<int, 6>{}, 8);
+  halve(std::integral_constant<int, 3>{}, 4);
+  halve(std::integral_constant<int, 2>{}, 2);
+  halve(std::integral_constant<int, 1>{}, 1);
+  // the lanes whose value is real, down the same splits: 3 → 2 | 1, 2 → 1 | 1 and 1 → 1 | 0, 1 → 1 | 0
+  if (!(lane & 1) && (lane & 6) != 6) atomicAdd(out + at, v[0]);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
-    k_gram(const TrackDesc<T>* __restrict__ D, const int* __restrict__ pre, const long long* __restrict__ wpre,
+    k_gram(const TrackDesc<T>* __restrict__ D, const int* pre, const long long* wpre,
            int ntracks, int par, int nmax, int R, int stages, int* __restrict__ err, uint64_t wait_ns) {
   using C = cplx<T>;
   using Cfg = GramCfg<T>;
@@ -250,6 +299,8 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
     for (int q = 0; q < stages; ++q) { mbar_init(&full[q], 1); mbar_init(&empty[q], Cfg::NCW); }
     mbar_init_fence();
   }
+  __shared__ PrefixSh psh;
+  stage_prefixes(psh, pre, wpre, ntracks);
   __syncthreads();
   TileWalk w;
   w.start(pre, wpre, ntracks, R, GRAM_TRACK_COST);
@@ -272,7 +323,7 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
       C* st = stage0 + (size_t)q * sel;
-      const int nz = Cfg::n4(n);
+      const int nz = Cfg::nr(n);
       for (int c = lane; c < 2 * n; c += 32) {
         const int l = c < n ? c : c - n;
         const C* src = (c < n ? d.Y[par] : d.AY[par]) + (size_t)z_phys(s, M, l) * d.n2 + r0;
@@ -288,7 +339,7 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
           pipe_fail(err, PIPE_DRAIN_TIMEOUT);
     return;
   }
-  // ---- consumers: thread (item, sub) accumulates one 4×4 block over rows sub, sub+split, …
+  // ---- consumers: thread (item, sub) accumulates one block of G and S over rows sub, sub+split, …
   constexpr int NC = Cfg::NCW * 32;
   const int tid = threadIdx.x;
   double2* red = reinterpret_cast<double2*>(smem_raw + 128 + (size_t)stages * sel * sizeof(C));
@@ -306,9 +357,9 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
   // with one or two rows each.
   constexpr bool COMP = sizeof(T) == 4;
   constexpr int GRAM_FOLD_ROWS = 16;
-  C acc[4][4], lo[COMP ? 4 : 1][COMP ? 4 : 1], t[COMP ? 4 : 1][COMP ? 4 : 1];
+  C acc[GRAM_E], lo[COMP ? GRAM_E : 1], t[COMP ? GRAM_E : 1];
   int tcnt = 0;
-  int cur = -1, items = 0, split = 1, nblk = 0, nb4 = 1, n = 0, item = 0, sub = 0, which = 0, bi = 0, bj = 0;
+  int cur = -1, items = 0, split = 1, nb = 1, n = 0, item = 0, sub = 0, bi = 0, bj = 0;
   bool active = false;
   for (; w.valid(); w.next()) {
     const TrackDesc<T>& d = D[w.t];
@@ -316,23 +367,18 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
       cur = w.t;
       const TrackState& s = *d.st;
       n = d.M + s.nWa + s.nP;
-      nb4 = (n + 3) / 4;
-      nblk = nb4 * (nb4 + 1) / 2;
-      items = 2 * nblk;
+      nb = gram_nb(n);
+      items = gram_items(n);
       split = max(1, NC / items);
       item = tid / split;
       sub = tid - item * split;
       active = item < items;
-      gram_item(active ? item : 0, nblk, nb4, which, bi, bj);
+      gram_item(active ? item : 0, nb, bi, bj);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = mk<C>(0, 0);
+      for (int e = 0; e < GRAM_E; ++e) acc[e] = mk<C>(0, 0);
       if constexpr (COMP) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) { lo[i][j] = mk<C>(0, 0); t[i][j] = mk<C>(0, 0); }
+        for (int e = 0; e < GRAM_E; ++e) lo[e] = t[e] = mk<C>(0, 0);
         tcnt = 0;
       }
     }
@@ -343,8 +389,9 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
     if (!failed) {
       if (active) {
         const C* st = stage0 + (size_t)q * sel;
-        const C* za = st + (size_t)(4 * bi) * CS;
-        const C* zb = st + (size_t)((which ? Cfg::n4(n) : 0) + 4 * bj) * CS;
+        const C* za = st + (size_t)(GRAM_B * bi) * CS;
+        const C* zb = st + (size_t)(GRAM_B * bj) * CS;
+        const C* zc = zb + (size_t)Cfg::nr(n) * CS;
         if constexpr (COMP) {
           const int mine = rows > sub ? (rows - sub + split - 1) / split : 0;
           if (tcnt > 0 && tcnt + mine > GRAM_FOLD_ROWS) {
@@ -352,34 +399,30 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
             tcnt = 0;
           }
           tcnt += mine;
-#pragma unroll 2
-          for (int r = sub; r < rows; r += split) {
-            C a[4], b[4], bs[4];
+        }
+#pragma unroll 1
+        for (int r = sub; r < rows; r += split) {
+          C a[GRAM_B], b[2 * GRAM_B];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { a[i] = za[i * CS + r]; b[i] = zb[i * CS + r]; }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bs[j] = make_float2(b[j].y, b[j].x);
+          for (int i = 0; i < GRAM_B; ++i) { a[i] = za[i * CS + r]; b[i] = zb[i * CS + r]; b[GRAM_B + i] = zc[i * CS + r]; }
+          if constexpr (COMP) {
             // conj(a)·b = a.x·(b.x, b.y) + a.y·(b.y, −b.x): two packed FP32x2 FMAs per product
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float2 ax = make_float2(a[i].x, a[i].x), ay = make_float2(a[i].y, -a[i].y);
+            for (int j = 0; j < 2 * GRAM_B; ++j) {
+              const float2 bs = make_float2(b[j].y, -b[j].x);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                t[i][j] = __ffma2_rn(ax, b[j], t[i][j]);
-                t[i][j] = __ffma2_rn(ay, bs[j], t[i][j]);
+              for (int i = 0; i < GRAM_B; ++i) {
+                float2& o = t[i * 2 * GRAM_B + j];
+                o = __ffma2_rn(make_float2(a[i].x, a[i].x), b[j], o);
+                o = __ffma2_rn(make_float2(a[i].y, a[i].y), bs, o);
               }
             }
-          }
-        } else {
-#pragma unroll 2
-          for (int r = sub; r < rows; r += split) {
-            C a[4], b[4];
+          } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { a[i] = za[i * CS + r]; b[i] = zb[i * CS + r]; }
+            for (int i = 0; i < GRAM_B; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-              for (int j = 0; j < 4; ++j) acc[i][j] = cmacc(acc[i][j], a[i], b[j]);  // conj(a)·b
+              for (int j = 0; j < 2 * GRAM_B; ++j)
+                acc[i * 2 * GRAM_B + j] = cmacc(acc[i * 2 * GRAM_B + j], a[i], b[j]);  // conj(a)·b
           }
         }
       }
@@ -390,43 +433,36 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
     if (w.last_of_track()) {
       // the split partial sums of each item meet in shared memory (FP64), then one global
       // atomic per matrix entry.  The split threads of an item are a contiguous run of lanes
-      // (item = tid / split), so each warp first sums its part of every run with a segmented
-      // shuffle (suffix sums toward the run's first lane; every lane of the warp takes part,
-      // idle ones with zeros) and only that first lane adds to shared memory: a few adds per
-      // entry instead of `split` (up to 80) contending ones.
+      // (item = tid / split): a warp sums its part of each of its items in turn (one or two of them for
+      // bases up to n = 15), the lanes of other items taking part with zeros.
       if constexpr (COMP) {
         if (active && tcnt > 0) gram_fold(acc, lo, t);
       }
-      {
-        const int key = active ? item : -1;
-        const unsigned seg = __match_any_sync(0xffffffffu, key);
-        const int head = __ffs(seg) - 1;
+      for (unsigned todo = __ballot_sync(0xffffffffu, active); todo;) {
+        const int it = __shfl_sync(0xffffffffu, item, __ffs(todo) - 1);
+        const bool mine = active && item == it;
+        todo &= ~__ballot_sync(0xffffffffu, mine);
+        static_assert(2 * GRAM_E % GRAM_SUM == 0, "whole groups");
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int g = 0; g < 2 * GRAM_E / GRAM_SUM; ++g) {
+          double v[GRAM_SUM];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            double vx = 0.0, vy = 0.0;
-            if (active) {
-              vx = (double)acc[i][j].x;
-              vy = (double)acc[i][j].y;
-              if constexpr (COMP) { vx += (double)lo[i][j].x; vy += (double)lo[i][j].y; }
-            }
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-              const double tx = __shfl_down_sync(0xffffffffu, vx, o), ty = __shfl_down_sync(0xffffffffu, vy, o);
-              if (lane + o < 32 && ((seg >> (lane + o)) & 1u)) { vx += tx; vy += ty; }
-            }
-            if (active && lane == head) {
-              atomicAdd(&red[item * 16 + i * 4 + j].x, vx);
-              atomicAdd(&red[item * 16 + i * 4 + j].y, vy);
-            }
+          for (int e = 0; e < GRAM_SUM / 2; ++e) {
+            const int x = g * (GRAM_SUM / 2) + e;
+            double re = (double)acc[x].x, im = (double)acc[x].y;
+            if constexpr (COMP) { re += (double)lo[x].x; im += (double)lo[x].y; }
+            v[2 * e] = mine ? re : 0.0;
+            v[2 * e + 1] = mine ? im : 0.0;
           }
+          gram_warp_sum(v, lane, reinterpret_cast<double*>(red + it * GRAM_E) + g * GRAM_SUM);
+        }
       }
       bar_sync_count(1, NC);
-      for (int e = tid; e < items * 16; e += NC) {
-        int wh, ei, ej;
-        gram_item(e >> 4, nblk, nb4, wh, ei, ej);
-        const int a = 4 * ei + ((e >> 2) & 3), b = 4 * ej + (e & 3);
+      for (int e = tid; e < items * GRAM_E; e += NC) {
+        int ei, ej;
+        gram_item(e / GRAM_E, nb, ei, ej);
+        const int i = e % GRAM_E / (2 * GRAM_B), j = e % (2 * GRAM_B), wh = j / GRAM_B;
+        const int a = GRAM_B * ei + i, b = GRAM_B * ej + (j - wh * GRAM_B);
         const double2 v = red[e];
         if (!failed && a < n && b < n && a <= b) {
           double2* g = d.gram_acc + (size_t)wh * NMAX * NMAX + (size_t)a * NMAX + b;
@@ -617,7 +653,7 @@ __device__ __forceinline__ void update_tile(const TrackDesc<T>& d, const TrackSt
 // MB: the largest block size of the launch (the tile bodies for M ≤ MB are compiled in).
 template <typename T, int MB>
 __global__ void __launch_bounds__(UpdCfg<T>::NT, 1)
-    k_update(const TrackDesc<T>* __restrict__ D, const int* __restrict__ pre, const long long* __restrict__ wpre,
+    k_update(const TrackDesc<T>* __restrict__ D, const int* pre, const long long* wpre,
              int ntracks, int par, IterParams prm, unsigned* __restrict__ ticket, int* __restrict__ err,
              uint64_t wait_ns) {
   using C = cplx<T>;
@@ -632,6 +668,8 @@ __global__ void __launch_bounds__(UpdCfg<T>::NT, 1)
     for (int q = 0; q < S; ++q) { mbar_init(&full[q], 1); mbar_init(&empty[q], Cfg::NCW); }
     mbar_init_fence();
   }
+  __shared__ PrefixSh psh;
+  stage_prefixes(psh, pre, wpre, ntracks);
   __syncthreads();
   TileWalk w;
   w.start(pre, wpre, ntracks, R);

@@ -240,3 +240,20 @@ def test_long_lines(omb, prec, Nx, Ny):
     scale = np.abs(op.HMkH(H[:, 0])) + k  # HMₖH of a random vector nearly cancels; compare on the operator's scale
     assert np.max(np.abs(omb.HMkH(k, ei, g, H, precision=prec) - ref)) < TOL[prec] * scale * 40
     assert rel(omb.E_field(k, ei, g, H[:, 0], precision=prec), O.E_field(k, H[:, 0], ei, O.Grid(6.0, 4.0, Nx, Ny))) < TOL[prec]
+
+
+@pytest.mark.parametrize("prec,tol", [("fp32", 5e-7), ("fp64", 1e-13)])
+@pytest.mark.parametrize("n2,n", [(2, 1), (96, 2), (192, 4), (768, 7), (1000, 15), (998, 16), (4096, 23), (514, 33), (2050, 36)])
+def test_gram_block_edges(omb, prec, tol, n2, n):
+    """Gram blocks of every remainder of the 3-wide column blocks, from one item to the largest basis
+    (so from 480 threads to 6 per item, warps of one, two and several items), and row counts below, at
+    and above a tile: within the bounds of test_gram_blocks_accuracy, relative to ‖z_a‖‖z_b‖."""
+    from omb200.ops import gram_blocks
+    rng = np.random.default_rng(n2 + n)
+    f32 = lambda: (rng.standard_normal((n2, n)) + 1j * rng.standard_normal((n2, n))).astype(np.complex64).astype(np.complex128)
+    Z, AZ = f32(), f32()
+    G, S = gram_blocks(Z, AZ, prec)
+    nz, na = np.linalg.norm(Z, axis=0), np.linalg.norm(AZ, axis=0)
+    up = np.triu(np.ones((n, n), dtype=bool))
+    assert np.max((np.abs(G - Z.conj().T @ Z) / np.outer(nz, nz))[up]) < tol
+    assert np.max((np.abs(S - Z.conj().T @ AZ) / np.outer(nz, na))[up]) < tol
