@@ -484,14 +484,14 @@ __device__ __forceinline__ void finish(TrackState& s, int status) {
   s.op_ncol = 0; s.pw_ncol = 0; s.hmkh_ncol = 0;
 }
 
-// The decisions after an update, for one track (one thread): residual norms from the sums of
-// k_update (cleared for the next iteration), locking, the phase's exits, and whether a Newton step
+// The decisions after an update, for one track (one thread): residual norms from the sums `ra` of
+// k_update, locking, the phase's exits, and whether a Newton step
 // is due.
-__device__ inline void control_track(TrackState& s, double* ra, const IterParams& prm) {
+__device__ inline void control_track(TrackState& s, const double* ra, const IterParams& prm) {
   if (s.done) return;
   const int M = s.M;
   double rs[MMAX];
-  for (int m = 0; m < M; ++m) { rs[m] = __ldcg(ra + m); ra[m] = 0.0; }
+  for (int m = 0; m < M; ++m) rs[m] = ra[m];
   bool bad = false;
   for (int m = 0; m < M; ++m) {
     s.resid[m] = sqrt(rs[m]);
@@ -765,7 +765,27 @@ __global__ void __launch_bounds__(UpdCfg<T>::NT, 1)
   if (last) {
     __threadfence();
     if (threadIdx.x == 0) *ticket = 0;
-    for (int t = threadIdx.x; t < ntracks; t += Cfg::NT) control_track(*D[t].st, D[t].res_acc, prm);
+    // a warp per track, on a copy of its state in shared memory: the decisions are a chain of dependent
+    // reads, one round trip to L2 this way.  (Read past L1, which may hold lines from before other CTAs'
+    // writes.)
+    __shared__ TrackState ctl[Cfg::NCW];
+    __shared__ double cres[Cfg::NCW][MMAX];
+    static_assert(sizeof(TrackState) % 8 == 0, "copied as 8-byte words");
+    constexpr int WORDS = (int)(sizeof(TrackState) / 8);
+    for (int t = warp; warp < Cfg::NCW && t < ntracks; t += Cfg::NCW) {
+      unsigned long long* g = reinterpret_cast<unsigned long long*>(D[t].st);
+      unsigned long long* c = reinterpret_cast<unsigned long long*>(&ctl[warp]);
+      double* ra = D[t].res_acc;
+      for (int i = lane; i < WORDS; i += 32) c[i] = __ldcg(g + i);
+      if (lane < MMAX) cres[warp][lane] = __ldcg(ra + lane);
+      __syncwarp();
+      if (ctl[warp].done) continue;
+      if (lane == 0) control_track(ctl[warp], cres[warp], prm);
+      __syncwarp();
+      if (lane < MMAX) ra[lane] = 0.0;
+      for (int i = lane; i < WORDS; i += 32) g[i] = c[i];
+      __syncwarp();
+    }
   }
 }
 
