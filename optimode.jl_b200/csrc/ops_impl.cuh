@@ -220,7 +220,7 @@ template <> const double2* tw_for<double>(const TwTables& t, int L) { return t.f
 
 template <typename T>
 static cudaError_t row_in(int mode, const OpUnit<T>* u, int nunits, int Nx, int Ny, int maxcol,
-                          const TwTables& t, cudaStream_t st, int gv = 1) {
+                          const TwTables& t, cudaStream_t st, int gv = TileChoice{}.row) {
   switch (Nx) {
 #define OMB_CASE(L) case L: return row_in_nx<T, L>(mode, u, nunits, Ny, maxcol, tw_for<T>(t, L), st, gv);
     OMB_FFT_SIZES(OMB_CASE)
@@ -230,7 +230,7 @@ static cudaError_t row_in(int mode, const OpUnit<T>* u, int nunits, int Nx, int 
 }
 template <typename T>
 static cudaError_t row_out(int mode, const OpUnit<T>* u, int nunits, int Nx, int Ny, int maxcol,
-                           const TwTables& t, cudaStream_t st, int gv = 1) {
+                           const TwTables& t, cudaStream_t st, int gv = TileChoice{}.row) {
   switch (Nx) {
 #define OMB_CASE(L) case L: return row_out_nx<T, L>(mode, u, nunits, Ny, maxcol, tw_for<T>(t, L), st, gv);
     OMB_FFT_SIZES(OMB_CASE)
