@@ -221,3 +221,17 @@ def test_rayleigh_ritz_block_sizes(omb, case, nev):
     assert np.allclose(ev, ref[:nev], rtol=1e-9, atol=0)
     V = np.stack(evecs, axis=1)
     assert np.allclose(V.conj().T @ V, np.eye(nev), atol=1e-10)
+
+
+def test_more_tracks_than_a_scan(omb, case):
+    """270 problems of two bands: 540 tracks, 270 per lane, so the live-tile prefixes take two rounds of
+    the 256-thread scan and are too many for the streaming kernels' shared-memory copy.  Every band
+    converges, and a sample agrees with the same problems solved alone (k rtol 1e-9)."""
+    grid, ei, _, _ = case
+    g = omb.Grid(6.0, 4.0, 24, 16)
+    om = OMEGA0 * (1 + 0.0005 * np.arange(270))
+    res, info = omb.solve_k_batch([{"omega": w, "eps_inv": ei, "grid": g, "nev": 2} for w in om], return_info=True)
+    assert all(np.all(i["status"] == 0) for i in info)
+    for j in (0, 1, 134, 135, 255, 256, 269):
+        km, _ = omb.solve_k(om[j], ei, g, nev=2)
+        assert np.allclose(res[j][0], km, rtol=1e-9, atol=0)
