@@ -275,18 +275,25 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
   const size_t gred = GramCfg<T>::red_entries(nmax) * sizeof(double2);
   const int gstages = (int)std::max<size_t>(2, std::min<size_t>(8, (200 * 1024 - 128 - gred) / gstage));
   const size_t sm_gram = 128 + gstages * gstage + gred;
-  const size_t sm_upd = UpdCfg<T>::smem;
   const size_t sm_rr = rr_smem(nmax);
   OMB_CU(set_smem(k_gram<T>, sm_gram));
-  auto update_kernel = Mmax <= 2 ? k_update<T, 2>
-                       : Mmax <= 4 ? k_update<T, 4>
-                       : Mmax <= 6 ? k_update<T, 6>
-                       : Mmax <= 8 ? k_update<T, 8> : k_update<T, MMAX>;
-  OMB_CU(set_smem(update_kernel, sm_upd));
+  // the update compiled for the smallest sufficient block size, with its tile shape
+  struct Upd { decltype(&k_update<T, 2>) kernel; int R, NT; size_t smem; };
+  auto upd_for = [](auto mb) {
+    using U = UpdCfg<T, decltype(mb)::value>;
+    return Upd{k_update<T, decltype(mb)::value>, U::R, U::NT, U::smem};
+  };
+  const Upd upd = Mmax <= 2   ? upd_for(std::integral_constant<int, 2>{})
+                  : Mmax <= 4 ? upd_for(std::integral_constant<int, 4>{})
+                  : Mmax <= 5 ? upd_for(std::integral_constant<int, 5>{})
+                  : Mmax <= 6 ? upd_for(std::integral_constant<int, 6>{})
+                  : Mmax <= 8 ? upd_for(std::integral_constant<int, 8>{})
+                              : upd_for(std::integral_constant<int, MMAX>{});
+  OMB_CU(set_smem(upd.kernel, upd.smem));
   OMB_CU(set_smem(k_rr, sm_rr));
   int occ_g = 0, occ_u = 0;
   OMB_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k_gram<T>, GramCfg<T>::NT, sm_gram));
-  OMB_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, update_kernel, UpdCfg<T>::NT, sm_upd));
+  OMB_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, upd.kernel, upd.NT, upd.smem));
   const int grid_g = std::max(1, occ_g) * ctx_->num_sms;
   const int grid_u = std::max(1, occ_u) * ctx_->num_sms;
   OMB_CU(gram_acc_.zero());
@@ -389,7 +396,7 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
         }))
       return e;
     k_newton<<<1, NEWTON_NT, 0, s>>>(d_state_ptrs_.p + a, d_hmkh_ptrs_.p + a, d_hmkh_nb_.p + a, d_n2_.p + a, n, rg,
-                                     UpdCfg<T>::R, preg, preu, wpreg, wpreu, prm);
+                                     upd.R, preg, preu, wpreg, wpreu, prm);
     if (!ok("k_newton", cudaGetLastError())) return e;
     if (!for_groups("operator pass", [&](const Group& g, int off, int cnt, cudaStream_t gs) {
           return op(OP_M, d_uA[par], off, cnt, g, 3 * g.Mmax, gs);
@@ -401,8 +408,8 @@ int Engine::run_phase(int phase, bool last, double tau, double lock_tol, int mod
     k_rr<<<n, RR_NT, sm_rr, s>>>(d_state_ptrs_.p + a, d_gram_ptrs_.p + a, d_coef_ptrs_.p + a, d_coef32_ptrs_.p + a, n,
                                  nmax, prm);
     if (!ok("k_rr", cudaGetLastError())) return e;
-    update_kernel<<<grid_u, UpdCfg<T>::NT, sm_upd, s>>>(d_descs.p + a, preu, wpreu, n, par, prm, d_ticket_.p + L,
-                                                        d_err_.p, ctx_->wait_ns);
+    upd.kernel<<<grid_u, upd.NT, upd.smem, s>>>(d_descs.p + a, preu, wpreu, n, par, prm, d_ticket_.p + L,
+                                                d_err_.p, ctx_->wait_ns);
     ok("k_update", cudaGetLastError());
     return e;
   };

@@ -552,10 +552,16 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
 // per tile row; a stage holds LG columns of Z and AZ for the tile plus the matching rows
 // of C and CP (in the block's precision), so the coefficients follow the tile's track.
 static_assert(MMAX == 12, "k_update dispatches M = 1..12");
-template <typename T> struct UpdCfg {
-  // rows per tile = consumer threads; with the producer warp 16 warps (FP32, 128 registers)
-  // or 9 warps (FP64, whose M ≤ 6 tile bodies need ≈170 registers)
-  static constexpr int R = sizeof(T) == 4 ? 480 : 256;
+template <typename T, int MB> struct UpdCfg {
+  // rows per tile = consumer threads.  FP32: 15 consumer warps in one CTA per SM (16 warps, 128
+  // registers).  FP64: 7 consumer warps; with the producer 8 warps, which leaves a thread 255 registers
+  // in one CTA per SM (blocks of 7 and 9 columns: 86.9 → 86.2 and 167.0 → 164.4 ms for a solve of a 512×256
+  // slot row, against 8 consumer warps whose 168 registers spill) and 128 in two.  Blocks of up to 6
+  // columns run two CTAs, so that one tile's stores (half of its bytes) overlap the other's loads and
+  // products: the sweep of twelve 256² instances 292.3 → 275.7 ms, a 512² solve 89.9 → 86.6, against one
+  // CTA of 256 rows (two CTAs of 128, 160 and 192 rows: 0.99, 1.04 and 1.05–1.06 of its speed on the sweep).
+  static constexpr int R = sizeof(T) == 4 ? 480 : 224;
+  static constexpr int CTAS = sizeof(T) == 8 && MB <= 6 ? 2 : 1;  // per SM
   static constexpr int LG = sizeof(T) == 4 ? 4 : 2;      // columns per stage
   static constexpr int NCW = R / 32;
   static constexpr int NT = (NCW + 1) * 32;
@@ -574,7 +580,7 @@ __device__ __forceinline__ void update_tile(const TrackDesc<T>& d, const TrackSt
                                             uint64_t* empty, int& q, uint32_t& ph, bool& failed,
                                             double (&racc)[MB], int* err, uint64_t wait_ns) {
   using C = cplx<T>;
-  using Cfg = UpdCfg<T>;
+  using Cfg = UpdCfg<T, MB>;
   constexpr int R = Cfg::R, LG = Cfg::LG, S = Cfg::STAGES;
   const int r = threadIdx.x, lane = r & 31;
   const int n = M + s.nWa + s.nP, nPn = s.nP_next;
@@ -652,12 +658,12 @@ __device__ __forceinline__ void update_tile(const TrackDesc<T>& d, const TrackSt
 
 // MB: the largest block size of the launch (the tile bodies for M ≤ MB are compiled in).
 template <typename T, int MB>
-__global__ void __launch_bounds__(UpdCfg<T>::NT, 1)
+__global__ void __launch_bounds__(UpdCfg<T, MB>::NT, UpdCfg<T, MB>::CTAS)
     k_update(const TrackDesc<T>* __restrict__ D, const int* pre, const long long* wpre,
              int ntracks, int par, IterParams prm, unsigned* __restrict__ ticket, int* __restrict__ err,
              uint64_t wait_ns) {
   using C = cplx<T>;
-  using Cfg = UpdCfg<T>;
+  using Cfg = UpdCfg<T, MB>;
   constexpr int R = Cfg::R, LG = Cfg::LG, S = Cfg::STAGES;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);
