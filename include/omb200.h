@@ -356,6 +356,16 @@ int omb_profile_apply(omb_ctx* ctx, int op, int precision, const omb_grid* grid,
 int omb_gram_blocks(omb_ctx* ctx, int precision, int64_t n2, int32_t n, const double* Z, const double* AZ,
                     double* G, double* S);
 
+/* The eigensolver's Rayleigh–Ritz step on caller Gram matrices: the lowest m (≤ 12) pairs of
+ * S c = λ G c for n×n (n ≤ 36) Hermitian G and S (host ComplexF64, column-major; the upper triangles
+ * are read), by the same kernel as a LOBPCG iteration.  precision chooses its tolerances (FP32
+ * or FP64 blocks; the arithmetic of the step is the same).  C receives n×m ComplexF64, column-major,
+ * CᴴGC = 1; lam the m ascending Ritz values; rank (may be NULL) the directions kept.  A G with
+ * fewer than m independent directions is OMB_ERR_ORTHO_FAIL; a non-finite S gives non-finite results.
+ * No reference counterpart (accuracy check; the reference calls LAPACK, ME/src/solvers/dftk.jl:304-506). */
+int omb_rayleigh_ritz(omb_ctx* ctx, int precision, int32_t n, int32_t m, const double* G, const double* S,
+                      double* C, double* lam, int32_t* rank);
+
 /* ---------------------------------------------------------------------------------
  * Kottke sub-pixel smoothing (the solver's input generator, lib/DielectricSmoothing)
  * --------------------------------------------------------------------------------- */

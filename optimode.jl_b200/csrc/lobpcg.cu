@@ -230,13 +230,8 @@ __global__ void __launch_bounds__(RR_NT) k_rr(TrackState* const* __restrict__ st
     Ev = V;
   }
   __syncthreads();
-  // ascending Ritz values
-  if (tid < r) {
-    const double d = lam[tid];
-    int at = 0;
-    for (int j = 0; j < r; ++j) at += lam[j] < d || (lam[j] == d && j < tid);
-    order[at] = tid;
-  }
+  // ascending Ritz values (non-finite ones, which end the track after the update, have a place too)
+  if (tid < r) order[rank_of([&](int j) { return lam[j]; }, r, tid)] = tid;
   __syncthreads();
   // coefficients of the new X in the Z columns (D L⁻ᴴ U, or D B U), and of the new P for the active
   // columns: the W and P parts of the Ritz vectors

@@ -85,6 +85,12 @@ struct IterParams {
   double jacobi_tol2;  // k_rr's Jacobi stops at ‖offdiag‖²_F ≤ jacobi_tol2·‖A‖²_F
   int maxiter, max_newton, last_phase, prec_diag;
 };
+// k_rr's tolerances for FP32 and FP64 blocks (an FP32 block's Gram matrices carry FP32 products:
+// rotating below 1e-9 of ‖A‖ buys nothing)
+inline void rr_tolerances(bool fp32, IterParams& prm) {
+  prm.gram_drop = fp32 ? 1e-6 : 1e-12;
+  prm.jacobi_tol2 = fp32 ? 1e-18 : 1e-26;
+}
 
 __device__ __forceinline__ int z_phys(const TrackState& s, int M, int l) {
   if (l < M) return l;

@@ -15,6 +15,8 @@
 // would never pass) or after `max_sweeps`.
 #pragma once
 
+#include <cmath>
+
 #include "omb_common.cuh"
 
 namespace omb {
@@ -135,6 +137,21 @@ __device__ inline void jacobi_eigh(double2* A, double2* V, int n, int ld, double
   }
   for (int e = tid; e < n; e += nt) A[e * ld + e].y = 0.0;
   __syncthreads();
+}
+
+// Position of entry i of the n values at(0), …, at(n − 1) in ascending order, ties by index and NaNs
+// counted as +∞: the positions are a permutation of 0..n−1 whatever the values are, so an index read
+// back from a table filled by them is always one of the n.
+template <typename F> __host__ __device__ __forceinline__ int rank_of(const F& at, int n, int i) {
+  using V = decltype(at(0));
+  auto key = [&](int j) { const V v = at(j); return v == v ? v : (V)INFINITY; };
+  const V d = key(i);
+  int r = 0;
+  for (int j = 0; j < n; ++j) {
+    const V e = key(j);
+    r += e < d || (e == d && j < i);
+  }
+  return r;
 }
 
 // ---- FP32 Jacobi refined to FP64 ------------------------------------------------------------
@@ -345,15 +362,7 @@ __device__ inline int eigh_refined(int oT, int oX, int oY, int oW, int n, int M,
   const float2* D = A + at;
   V += at;
   // ascending order of the FP32 eigenvalues (the padding stays at index n)
-  if (tid < n) {
-    const float d = D[tid * ldf + tid].x;
-    int rank = 0;
-    for (int j = 0; j < n; ++j) {
-      const float dj = D[j * ldf + j].x;
-      rank += dj < d || (dj == d && j < tid);
-    }
-    order[rank] = tid;
-  }
+  if (tid < n) order[rank_of([&](int j) { return D[j * ldf + j].x; }, n, tid)] = tid;
   __syncthreads();
   for (int i = ty; i < n; i += 16)
     for (int j = tx; j < n; j += 16) {

@@ -28,7 +28,7 @@ OPS = {"M": 0, "P": 1, "P_diag": 2}
 #: every symbol ``include/omb200.h`` declares (checked by the CPU test suite)
 EXPORTS = (
     "omb_version", "omb_fft_size_supported", "omb_last_error", "omb_ctx_create",
-    "omb_ctx_destroy", "omb_apply", "omb_HMkH", "omb_efield", "omb_hfield", "omb_gram_blocks",
+    "omb_ctx_destroy", "omb_apply", "omb_HMkH", "omb_efield", "omb_hfield", "omb_gram_blocks", "omb_rayleigh_ritz",
     "omb_autotune", "omb_ctx_set_autotune", "omb_tune_set", "omb_tune_get", "omb_tune_clear", "omb_tune_save",
     "omb_tune_load",
 )
@@ -96,6 +96,8 @@ def load():
             "omb_efield": (ctypes.c_int, [vp, ctypes.c_int, gp, ctypes.c_double, _dp, _dp, _dp]),
             "omb_hfield": (ctypes.c_int, [vp, gp, ctypes.c_double, ctypes.c_int, _dp, _dp]),
             "omb_gram_blocks": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int64, ctypes.c_int32, _dp, _dp, _dp, _dp]),
+            "omb_rayleigh_ritz": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int32, ctypes.c_int32, _dp, _dp, _dp, _dp,
+                                                 ctypes.POINTER(ctypes.c_int32)]),
             "omb_autotune": (ctypes.c_int, [vp, gp, ctypes.c_int32] + [ctypes.POINTER(ctypes.c_int32)] * 3 + [_dp]),
             "omb_ctx_set_autotune": (ctypes.c_int, [vp, ctypes.c_int32]),
             "omb_tune_set": (ctypes.c_int, [ctypes.c_char_p] + [ctypes.c_int32] * 5),

@@ -121,6 +121,22 @@ def gram_blocks(Z, AZ, precision: str = "fp32", device: int = 0):
     return G, S
 
 
+def rayleigh_ritz(G, S, m: int, precision: str = "fp64", device: int = 0):
+    """(λ, C, rank): the lowest `m` pairs of S c = λ G c from the eigensolver's Rayleigh–Ritz kernel
+    (``omb_rayleigh_ritz``) for Hermitian (n, n) matrices, n ≤ 36."""
+    lib = _lib.load()
+    ctx = _lib.context(device)
+    G = np.asfortranarray(np.asarray(G, dtype=np.complex128))
+    S = np.asfortranarray(np.asarray(S, dtype=np.complex128))
+    n = G.shape[0]
+    C = np.zeros((n, m), dtype=np.complex128, order="F")
+    lam = np.zeros(m)
+    rank = ctypes.c_int32()
+    _lib.check(lib.omb_rayleigh_ritz(ctx.handle, _lib.PREC[precision], int(n), int(m), _dptr(G), _dptr(S), _dptr(C),
+                                     _dptr(lam), ctypes.byref(rank)))
+    return lam, C, rank.value
+
+
 # ---- operator-tile autotuning -------------------------------------------------------------
 
 def autotune(grid, ncol: int = 4, device: int = 0):
