@@ -59,7 +59,7 @@ template <typename T> __device__ __forceinline__ Basis<T> basis_pass(T k, T gx, 
   const T p2 = gx * gx + gy * gy, m2 = p2 + k * k;
   const T im = rsqrt_of(m2);
   b.imag = im;
-  b.mag = m2 * im;
+  b.mag = m2 == T(0) ? T(0) : m2 * im;  // (k + G = 0: k equal to a g_z of a z-periodic cell)
   if (p2 > T(0)) {
     const T ip = rsqrt_of(p2);
     const T kim = k * ip * im;

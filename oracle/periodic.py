@@ -64,7 +64,9 @@ def mag_mn(k: float, grid: Grid3):
     with np.errstate(invalid="ignore", divide="ignore"):
         n = np.where((perp > 0)[..., None], zxw / perp[..., None], np.array([0.0, 1.0, 0.0]))
     m = np.cross(n, w)
-    m = m / np.sqrt(np.sum(m * m, axis=-1))[..., None]
+    with np.errstate(invalid="ignore"):
+        # (w = 0, k equal to a g_z: the limit along +ẑ; mag = 0 takes the plane wave out of M̂ and HMₖH)
+        m = np.where((mag > 0)[..., None], m / np.sqrt(np.sum(m * m, axis=-1))[..., None], np.array([1.0, 0.0, 0.0]))
     return mag, m, n
 
 

@@ -66,6 +66,27 @@ def test_apply3_and_HMkH3_match_oracle(omb, prec, dims):
         assert abs(hm[j] - ref) <= 10 * TOL[prec] * np.linalg.norm(H[:, j]) ** 2 * 1.3
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("dims,slab", [((24, 16, 8), 1), ((24, 16, 8), 3), ((320, 8, 8), 1), ((12, 40, 12), 2)])
+def test_apply3_at_a_reciprocal_vector(omb, prec, dims, slab):
+    """k = g_z: one plane wave of the cell has k + G = 0.  Its |k + G| is zero, so M̂ and HMₖH do not see it;
+    both are finite and match the oracle, in every form of the row passes (FP64, FP32, long lines)."""
+    Nx, Ny, Nz = dims
+    L = 0.25
+    k = slab / L
+    ei = grating(Nx, Ny, Nz)
+    g = omb.Grid3(6.0, 4.0, L, Nx, Ny, Nz)
+    op = OP.Operator3(k, ei, OP.Grid3(6.0, 4.0, L, Nx, Ny, Nz))
+    assert op.mag[slab, 0, 0] == 0.0
+    rng = np.random.default_rng(6)
+    H = rng.standard_normal((op.size, 2)) + 1j * rng.standard_normal((op.size, 2))
+    got = omb.apply3("M", k, ei, g, H, precision=prec)
+    hm = omb.HMkH3(k, ei, g, H, precision=prec)
+    for j in range(2):
+        assert rel(got[:, j], op.M(H[:, j])) <= TOL[prec], j
+        assert abs(hm[j] - op.HMkH(H[:, j])) <= 10 * TOL[prec] * np.linalg.norm(H[:, j]) ** 2 * k
+
+
 def test_apply3_hermitian(omb):
     """⟨a|M̂b⟩ = conj⟨b|M̂a⟩ on the 3D operator (``ME/test/runtests.jl:58``)."""
     ei = grating()
