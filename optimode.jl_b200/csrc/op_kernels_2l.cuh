@@ -50,16 +50,24 @@ template <typename T> __host__ __device__ constexpr int l2_col_threads(int NY) {
 }
 
 // Transverse basis for the pass kernels (basis_at with 1/|k+G| and 1/|G| from reciprocal square
-// roots: ≤ 2 ulp; two such operations per pixel instead of two square roots and two divisions, which
-// in FP64 were more than half of a row pass's prologue).
+// roots: two such operations per pixel instead of two square roots and two divisions, which
+// in FP64 were more than half of a row pass's prologue).  m2·rsqrt(m2) rounds once more than √m2, and |k+G|
+// enters M̂ twice: the FP64 form takes the residual m2 − mag² back in (one Newton step of the square
+// root, three operations), without which M̂ was 3–5 % further from an extended-precision one than with
+// basis_at.
 __device__ __forceinline__ float rsqrt_of(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double rsqrt_of(double x) { return rsqrt(x); }
+__device__ __forceinline__ float root_from(float x, float r) { return x * r; }
+__device__ __forceinline__ double root_from(double x, double r) {
+  const double y = x * r;
+  return fma(fma(-y, y, x), 0.5 * r, y);
+}
 template <typename T> __device__ __forceinline__ Basis<T> basis_pass(T k, T gx, T gy) {
   Basis<T> b;
   const T p2 = gx * gx + gy * gy, m2 = p2 + k * k;
   const T im = rsqrt_of(m2);
   b.imag = im;
-  b.mag = m2 == T(0) ? T(0) : m2 * im;  // (k + G = 0: k equal to a g_z of a z-periodic cell)
+  b.mag = m2 == T(0) ? T(0) : root_from(m2, im);  // (k + G = 0: k equal to a g_z of a z-periodic cell)
   if (p2 > T(0)) {
     const T ip = rsqrt_of(p2);
     const T kim = k * ip * im;
