@@ -791,7 +791,9 @@ __global__ void __launch_bounds__(UpdCfg<T, MB>::NT, UpdCfg<T, MB>::CTAS)
       for (int i = lane; i < WORDS; i += 32) c[i] = __ldcg(g + i);
       if (lane < MMAX) cres[warp][lane] = __ldcg(ra + lane);
       __syncwarp();
-      if (ctl[warp].done) continue;
+      const bool over = ctl[warp].done;
+      __syncwarp();  // (every lane has read the flag before the warp's next track overwrites it)
+      if (over) continue;
       if (lane == 0) control_track(ctl[warp], cres[warp], prm);
       __syncwarp();
       if (lane < MMAX) ra[lane] = 0.0;
