@@ -162,7 +162,7 @@ bool tune_known(int dev, int Nx, int Ny) {
 }
 
 // Times the tile × wave variants (168 slots; each cluster apply once) of one FP32 M̂ application to `ncol` columns on `units`
-// copies of a uniform cell and records the fastest (ties: the fastest on one unit).
+// copies of a uniform cell and records the fastest.
 int autotune_grid(omb_ctx* ctx, const omb_grid* g, int ncol, int units, TileChoice* best, double* times) {
   int rc = check_grid(g);
   if (rc) return rc;
@@ -202,26 +202,6 @@ int autotune_grid(omb_ctx* ctx, const omb_grid* g, int ncol, int units, TileChoi
   double best_s = 1e30;
   TileChoice bt;
   rc = OMB_OK;
-  // seconds per application of variant (r, c, wv) to n units
-  auto time_variant = [&](int r, int c, int wv, int n, int reps, double& s) -> int {
-    {
-      std::lock_guard<std::mutex> lk(g_tune_mu);
-      ensure_loaded_locked();
-      g_tune[TuneKey{name, g->Nx, g->Ny}] = TuneEntry{r, c, 0.0, wv};
-    }
-    cudaError_t e = cudaSuccess;
-    for (int w = 0; w < 2 && e == cudaSuccess; ++w) e = launch_op<float>(OP_M, du.p, n, g->Nx, g->Ny, ncol, ctx->tw, st);
-    if (e == cudaSuccess) e = cudaEventRecord(e0, st);
-    for (int w = 0; w < reps && e == cudaSuccess; ++w) e = launch_op<float>(OP_M, du.p, n, g->Nx, g->Ny, ncol, ctx->tw, st);
-    if (e == cudaSuccess) e = cudaEventRecord(e1, st);
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-    float ms = 0;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-    if (e != cudaSuccess) return cuda_fail(e, "autotune");
-    s = ms * 1e-3 / reps;
-    return OMB_OK;
-  };
-  std::vector<std::pair<double, TileChoice>> all;
   int vi = 0;
   for (int r = 0; r < ROW_VARIANTS && !rc; ++r)
     for (int c = 0; c < COL_VARIANTS && !rc; ++c)
@@ -230,24 +210,25 @@ int autotune_grid(omb_ctx* ctx, const omb_grid* g, int ncol, int units, TileChoi
           if (times) times[vi] = -1.0;  // one kernel whatever the column and wave choices: timed once
           continue;
         }
-        double s = 0;
-        rc = time_variant(r, c, wv, units, 5, s);
-        if (rc) break;
+        {
+          std::lock_guard<std::mutex> lk(g_tune_mu);
+          ensure_loaded_locked();
+          g_tune[TuneKey{name, g->Nx, g->Ny}] = TuneEntry{r, c, 0.0, wv};
+        }
+        cudaError_t e = cudaSuccess;
+        for (int w = 0; w < 2 && e == cudaSuccess; ++w) e = launch_op<float>(OP_M, du.p, units, g->Nx, g->Ny, ncol, ctx->tw, st);
+        if (e == cudaSuccess) e = cudaEventRecord(e0, st);
+        const int reps = 5;
+        for (int w = 0; w < reps && e == cudaSuccess; ++w) e = launch_op<float>(OP_M, du.p, units, g->Nx, g->Ny, ncol, ctx->tw, st);
+        if (e == cudaSuccess) e = cudaEventRecord(e1, st);
+        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+        float ms = 0;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        if (e != cudaSuccess) { rc = cuda_fail(e, "autotune"); break; }
+        const double s = ms * 1e-3 / reps;
         if (times) times[vi] = s;
-        all.push_back({s, TileChoice{r, c, wv}});
-        best_s = std::min(best_s, s);
+        if (s < best_s) { best_s = s; bt.row = r; bt.col = c; bt.wave = wv; }
       }
-  // Under a full load the variants of small grids differ by less than the timing's noise, while on one
-  // unit (what a single solve launches) they differ by up to 1.5×: among those within TIE of the best
-  // the fastest on one unit is taken.
-  constexpr double TIE = 1.03;
-  double best_one = 1e30, best_all = best_s;
-  for (const auto& v : all) {
-    if (rc || v.first > TIE * best_all) continue;
-    double s = 0;
-    rc = time_variant(v.second.row, v.second.col, v.second.wave, 1, 10, s);
-    if (!rc && s < best_one) { best_one = s; bt = v.second; best_s = v.first; }
-  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   {
