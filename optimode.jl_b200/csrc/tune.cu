@@ -290,7 +290,9 @@ int omb_tune_get(const char* device_name, int32_t Nx, int32_t Ny, int32_t* row_v
   std::lock_guard<std::mutex> lk(g_tune_mu);
   ensure_loaded_locked();
   auto it = g_tune.find(TuneKey{device_name, Nx, Ny});
-  if (it == g_tune.end()) return fail(OMB_ERR_INVALID_ARG, "no tuned tiles for this device and grid");
+  // (an entry that the passes do not take is not in force)
+  if (it == g_tune.end() || it->second.stale)
+    return fail(OMB_ERR_INVALID_ARG, "no tuned tiles for this device and grid");
   if (row_variant) *row_variant = it->second.row;
   if (col_variant) *col_variant = it->second.col;
   if (wave_variant) *wave_variant = it->second.wave;
