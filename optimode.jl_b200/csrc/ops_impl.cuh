@@ -185,10 +185,12 @@ static cudaError_t col_ny(int mode, const OpUnit<T>* u, int nunits, int Nx, int 
                           const cplx<T>* tw, cudaStream_t st, int tv = 1) {
   if constexpr (sizeof(T) == 4) {
     // (lines above 256 points: one register budget for both component-parallel variants, and variant 5
-    // is the default tile)
-    if (mode == CM_M && tv == 5 && NY <= 256)
-      return col_b4<NY, CS_FWD, PW_EPS, CS_INV>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Nx, maxcol,
-                                                reinterpret_cast<const float2*>(tw), st);
+    // is the default tile: four CTAs per SM would spill)
+    if constexpr (NY <= 256) {
+      if (mode == CM_M && tv == 5)
+        return col_b4<NY, CS_FWD, PW_EPS, CS_INV>(reinterpret_cast<const OpUnit<float>*>(u), nunits, Nx, maxcol,
+                                                  reinterpret_cast<const float2*>(tw), st);
+    }
     if (mode == CM_M && (tv == 3 || tv == 4)) {
       const auto* uf = reinterpret_cast<const OpUnit<float>*>(u);
       const auto* tf = reinterpret_cast<const float2*>(tw);
