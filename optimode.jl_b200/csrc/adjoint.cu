@@ -439,11 +439,12 @@ static int pullback_impl(omb_ctx* ctx, Problem& P, double omega, int nev, const 
   OMB_CU(eib.zero());
   double wbar = 0.0, Lbar = 0.0;
   // The bands of a chunk run together: at a few hundred KB to a few MB per vector one band's launches
-  // leave most SMs idle.  A band holds 10 vectors and 6 planar fields (28·N complex numbers more than
-  // its inputs); a chunk is limited to 4 GiB of them.
-  const int chunk = (int)std::max<long long>(1, std::min<long long>(nev, ((long long)4 << 30) / (38 * N * (long long)sizeof(double2))));
-  for (int b0 = 0; b0 < nev; b0 += chunk) {
-    const int nb = std::min(chunk, nev - b0);
+  // leave most SMs idle.  A band holds up to 10 vectors and 6 planar fields (38·N complex numbers); a
+  // chunk is limited to 4 GiB of them, and to what a nearly full device still has (halved until its
+  // vectors and fields fit; one band needs no more than this).
+  int chunk = (int)std::max<long long>(1, std::min<long long>(nev, ((long long)4 << 30) / (38 * N * (long long)sizeof(double2))));
+  for (int b0 = 0, nb = 0; b0 < nev; b0 += nb) {
+    nb = std::min(chunk, nev - b0);
     // bands with a field cotangent (the others need no adjoint solve)
     std::vector<int> mb;  // MINRES index → band of the chunk
     for (int j = 0; j < nb && evbar; ++j) {
@@ -458,9 +459,16 @@ static int pullback_impl(omb_ctx* ctx, Problem& P, double omega, int nev, const 
     DevBuf<MinresState> S;
     DevBuf<unsigned> tick;
     DevBuf<AdjBand> dband;
-    OMB_CU(ev.alloc(n2 * nb, st));
-    OMB_CU(vecs.alloc(9 * n2 * nm, st));       // x v w w2 r1 r2 y Av b
-    OMB_CU(scr.alloc(6 * 3 * N * nb, st));
+    cudaError_t ae = ev.alloc(n2 * nb, st);
+    if (ae == cudaSuccess) ae = vecs.alloc(9 * n2 * nm, st);  // x v w w2 r1 r2 y Av b
+    if (ae == cudaSuccess) ae = scr.alloc(6 * 3 * N * nb, st);
+    if (ae == cudaErrorMemoryAllocation && nb > 1) {
+      cudaGetLastError();  // (a failed allocation leaves no other trace)
+      chunk = (nb + 1) / 2;
+      nb = 0;
+      continue;
+    }
+    OMB_CU(ae);
     OMB_CU(kd.alloc(nb, st));
     OMB_CU(hpart.alloc(2 * (size_t)rb * nb, st));
     OMB_CU(hred.alloc(4 * (size_t)nb, st));

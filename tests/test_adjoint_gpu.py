@@ -140,3 +140,42 @@ def test_bands_solved_together_equal_bands_alone(omb, nx, ny):
         w1, e1 = w1 + w, e1 + e
     assert np.isclose(wb, w1, rtol=1e-11, atol=0)
     assert _rel(eib, e1) < 1e-11
+
+
+_NEARLY_FULL = """
+import sys
+import numpy as np
+import torch
+import omb200 as omb
+d = np.load(sys.argv[1])
+g = omb.Grid(6.0, 4.0, 512, 512)
+omb.apply_M(1.0, d["ei"], g, d["kv"][0])  # the library's modules, tables and pools are in place
+torch.cuda.synchronize()
+left = int(sys.argv[2]) << 20
+hold = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+wb, eib = omb.pullback(float(d["w"]), d["ei"], g, d["km"], list(d["kv"]), list(d["kb"]))
+np.savez(sys.argv[3], wb=wb, eib=eib)
+"""
+
+
+def test_pullback_on_a_nearly_full_device(omb, tmp_path):
+    """Four bands of a 512² cell with 200 MiB of the device left: their fields alone take 302 MB beside
+    the cell's own arrays, so the bands run in smaller chunks, and the result is that of all four at
+    once (up to the rounding of the accumulation)."""
+    import os
+    import subprocess
+    import sys
+    from conftest import PKG
+    g = omb.Grid(6.0, 4.0, 512, 512)
+    ei = gaussian_epsinv(P_WG, Nx=512, Ny=512)
+    km, kv = omb.solve_k(OMEGA0, ei, g, nev=4)
+    kb = [0.3, -0.7, 0.2, 0.5]
+    wb, eib = omb.pullback(OMEGA0, ei, g, km, kv, kb)
+    np.savez(tmp_path / "in.npz", ei=ei, km=km, kv=np.stack(kv), kb=kb, w=OMEGA0)
+    env = dict(os.environ, PYTHONPATH=PKG)
+    r = subprocess.run([sys.executable, "-c", _NEARLY_FULL, str(tmp_path / "in.npz"), "200", str(tmp_path / "out.npz")],
+                       env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    out = np.load(tmp_path / "out.npz")
+    assert np.isclose(float(out["wb"]), wb, rtol=1e-11, atol=0)
+    assert _rel(out["eib"], eib) < 1e-11
