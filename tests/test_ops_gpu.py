@@ -257,3 +257,23 @@ def test_gram_block_edges(omb, prec, tol, n2, n):
     up = np.triu(np.ones((n, n), dtype=bool))
     assert np.max((np.abs(G - Z.conj().T @ Z) / np.outer(nz, nz))[up]) < tol
     assert np.max((np.abs(S - Z.conj().T @ AZ) / np.outer(nz, na))[up]) < tol
+
+
+@pytest.mark.parametrize("Nx,Ny", [(320, 12), (8, 320), (384, 20), (40, 384), (512, 24), (12, 512), (384, 320)])
+def test_long_line_tile_variants(omb, Nx, Ny):
+    """Every row and column variant that the autotuner may choose for lines above 256 points, beside short
+    lines that leave a remainder in its tiles: the FP32 M̂ within the tolerance of the default tiles' test."""
+    import torch
+    from omb200 import ops
+    name = torch.cuda.get_device_name(0)
+    g = omb.Grid(6.0, 4.0, Nx, Ny)
+    ei = random_epsinv(Nx, Ny, seed=Nx + 3 * Ny)
+    H = rand_block(2 * g.N, 2, seed=Ny)
+    ref = O.Operator(1.23, ei, O.Grid(6.0, 4.0, Nx, Ny)).M_block(H)
+    try:
+        for r in range(5):
+            for c in range(6):
+                ops.tune_set(name, Nx, Ny, r, c, 0)
+                assert rel(omb.apply_M(1.23, ei, g, H, precision="fp32"), ref) < TOL["fp32"], (r, c)
+    finally:
+        ops.tune_set(name, Nx, Ny, 1, 1, 0)
