@@ -490,6 +490,8 @@ __device__ __forceinline__ void finish(TrackState& s, int status) {
   s.op_ncol = 0; s.pw_ncol = 0; s.hmkh_ncol = 0;
 }
 
+constexpr int REFRESH = 8;  // iterations without a better residual after which AX and AP are recomputed
+
 // The decisions after an update, for one track (one thread): residual norms from the sums `ra` of
 // k_update, locking, the phase's exits, and whether a Newton step
 // is due.
@@ -545,6 +547,19 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
     if (maxres < prm.tol) s.hmkh_ncol = 1;
   }
   if (s.iter_phase >= prm.maxiter && s.hmkh_ncol == 0) { finish(s, last ? TS_MAXITER : TS_PHASE_DONE); return; }
+  // AX and AP are carried by their recurrences, whose rounding error grows where W and P are nearly
+  // parallel (residuals that rise steadily from ≈1e-11 in FP64, Ritz values below the spectrum in FP32).
+  // A track that has not improved for REFRESH iterations forms them afresh from X, W and P, all columns
+  // unlocked; a pending Newton step does so anyway.
+  if (s.hmkh_ncol == 0 && s.stall > 0 && s.stall % REFRESH == 0) {
+    s.nlocked = 0;
+    s.nWa = M;
+    s.op_col0 = 0;
+    s.op_ncol = 2 * M + s.nP;
+    s.pw_col0 = 0;
+    s.pw_ncol = M;
+    return;
+  }
   s.nWa = M - s.nlocked;
   s.op_col0 = M + s.nlocked;
   s.op_ncol = s.nWa;
