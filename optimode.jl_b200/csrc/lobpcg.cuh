@@ -548,14 +548,20 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
   }
   if (s.iter_phase >= prm.maxiter && s.hmkh_ncol == 0) { finish(s, last ? TS_MAXITER : TS_PHASE_DONE); return; }
   // AX and AP are carried by their recurrences, whose rounding error grows where W and P are nearly
-  // parallel (residuals that rise steadily from ≈1e-11 in FP64, Ritz values below the spectrum in FP32).
-  // A track that has not improved for REFRESH iterations forms them afresh from X, W and P, all columns
-  // unlocked; a pending Newton step does so anyway.
-  if (s.hmkh_ncol == 0 && s.stall > 0 && s.stall % REFRESH == 0) {
+  // parallel: residuals that rise steadily (from ≈1e-11 in FP64), Ritz values below the spectrum, or a
+  // zigzag on the few directions that the Gram floor leaves.  A track that has not improved for REFRESH
+  // iterations, or has a Ritz value that a positive operator cannot have, starts again from X: AX and AW
+  // formed afresh, no P, all columns unlocked.  (A pending Newton step recomputes them anyway, but takes
+  // no Ritz value from a broken block.  Of 360 starts of a 128² cell with two bands 4.5e-6 apart in k, 6
+  // stayed unconverged with P kept and none without.)
+  const bool broken = s.lam[0] <= 0.0;
+  if (broken) s.hmkh_ncol = 0;
+  if (broken || (s.hmkh_ncol == 0 && s.stall > 0 && s.stall % REFRESH == 0)) {
     s.nlocked = 0;
     s.nWa = M;
+    s.nP = 0;
     s.op_col0 = 0;
-    s.op_ncol = 2 * M + s.nP;
+    s.op_ncol = 2 * M;
     s.pw_col0 = 0;
     s.pw_ncol = M;
     return;

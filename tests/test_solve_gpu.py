@@ -242,17 +242,17 @@ NEAR_PAIR = ((3.554630006558236, 2.003322750103637, 0.4164621074304316, 0.486723
 
 
 def test_near_degenerate_pair_converges_from_any_start(omb):
-    """Two bands 4.5e-6 apart in k, to residuals of 3e-12 from different random blocks: the recurrences of
-    AX and AP lose accuracy while the pair separates, and without forming them afresh some starts end with
-    residuals of 1e-8 to 1e-5 that no longer fall (both operator precisions of the mixed solve)."""
+    """Two bands 4.5e-6 apart in k, to residuals of 3e-12 from 40 random blocks: the recurrences of
+    AX and AP lose accuracy while the pair separates, and without starting again from X about one start in
+    six ended with residuals of 1e-8 to 1e-5 that no longer fell."""
     P, w = NEAR_PAIR
     g = omb.Grid(3.0, 2.0, 128, 128)
     ei = gaussian_epsinv(P, 3.0, 2.0, 128, 128)
     ks = []
-    for seed in range(1, 13):
+    for seed in range(1, 41):
         km, _, info = omb.solve_k(w, ei, g, omb.B200Solver(precision="mixed", seed=seed), nev=4, k_tol=1e-12, eig_tol=3e-12,
                                   return_info=True)
-        assert np.all(info["status"] == 0) and np.max(info["iterations"]) < 500, (seed, info)
+        assert np.all(info["status"] == 0) and np.max(info["iterations"]) < 800, (seed, info)
         ks.append(km)
     # residual 3e-12: λ to 1e-12 or better, so k to 1e-11 whatever the start
     assert np.allclose(ks, ks[0], rtol=0, atol=1e-11)
