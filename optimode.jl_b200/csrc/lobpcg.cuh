@@ -540,6 +540,11 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
       const bool at_floor = maxres < 4.0 * prm.tau_phase;
       if (at_floor && s.stall >= 8) { finish(s, TS_PHASE_DONE); return; }
       if (s.newton_steps > 0 && s.stall >= 8) { finish(s, TS_PHASE_DONE); return; }
+      // k has settled to what FP32 resolves and the residual hovers between the floor and 4 × it: another
+      // step would move k by its noise only, and restart the count of stalled iterations
+      if (at_floor && s.newton_phase > 0 && s.stall >= 4 && fabs(s.dk_last) < prm.dk_phase) {
+        finish(s, TS_PHASE_DONE); return;
+      }
       if (s.since_newton >= 2 && (maxres < fmax(0.1 * fabs(dw2), prm.tau_phase) || (at_floor && s.stall >= 4)))
         s.hmkh_ncol = 1;
     }

@@ -256,3 +256,23 @@ def test_near_degenerate_pair_converges_from_any_start(omb):
         ks.append(km)
     # residual 3e-12: λ to 1e-12 or better, so k to 1e-11 whatever the start
     assert np.allclose(ks, ks[0], rtol=0, atol=1e-11)
+
+
+@pytest.mark.parametrize("seed", [20315, 21121, 23116])
+def test_fp32_phase_hands_over_at_its_floor(omb, seed):
+    """Frequency sweeps of a narrow LiNbO₃ ridge on 256², started by the learned network, whose FP32 residuals
+    settle just above the level that ends the FP32 phase: the phase ends once k has settled, instead of
+    taking Newton steps by the noise of k (40 to 60 of the 60 that a band has in most of these solves), so
+    that 10 steps in all are enough (5 are usual)."""
+    import importlib.util
+    import os
+    from conftest import ROOT
+    spec = importlib.util.spec_from_file_location("speed_cases", os.path.join(ROOT, "perf", "cases.py"))
+    cases = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(cases)
+    s = cases.prepare({"do": "sweep", "family": "ridge", "nx": 256, "ny": 256, "nev": 2, "widths": 1, "omegas": 4,
+                       "warm": "sweep_learned"}, seed)
+    for _ in range(8):
+        _, info = omb.solve_k_batch(s["problems"], s["solver"], k_tol=1e-12, eig_tol=3e-12, max_eigsolves=10, return_info=True)
+        for i in info:
+            assert np.all(i["status"] == 0) and np.max(i["newton_steps"]) <= 10
