@@ -436,14 +436,17 @@ __device__ inline int eigh_refined(int oT, int oX, int oY, int oW, int n, int M,
       }
     __syncthreads();
     bool more = false, bad = false;
+    // one thread per pair i < j: E_ji = conj(R_ij − E_ij), the same formula with S and R taken as exactly
+    // Hermitian.  (From the two roundings of S_ij and S_ji the columns of a pair would be orthogonal only to
+    // ε‖T‖/|λ_j − λ_i|: 1e-10 for a pair 1e-5 apart.)
 #pragma unroll
     for (int a = 0; a < TL; ++a)
 #pragma unroll
       for (int b = 0; b < TL; ++b) {
         const int i = ty + 16 * a, j = tx + 16 * b;
-        if (i >= n || j >= n) continue;
+        if (i > j || i >= n || j >= n) continue;
         const double2 s = t1[a][b], r = t2[a][b];
-        double2 e = make_double2(0.5 * r.x, 0.5 * r.y);
+        double2 e = make_double2(0.5 * r.x, i == j ? 0.0 : 0.5 * r.y);
         if (i != j) {
           const double lj = lam[j];
           const double inv = (double)__frcp_rn((float)(lj - lam[i]));  // (a relative error of 1e-7: 1e-15 in a last step)
@@ -451,13 +454,13 @@ __device__ inline int eigh_refined(int oT, int oX, int oY, int oW, int n, int M,
           const double f1 = fabs(f.x) + fabs(f.y);
           if (f1 <= E_MAX) e = f;             // (false for a NaN or infinite quotient)
           else if (i < M || j < M) bad = true;  // unwanted close pairs may stay mixed
-        } else {
-          e.y = 0;
         }
-        const double e1 = fabs(e.x) + fabs(e.y);
+        const double2 h = i == j ? e : make_double2(r.x - e.x, e.y - r.y);
+        const double e1 = fmax(fabs(e.x) + fabs(e.y), fabs(h.x) + fabs(h.y));
         if (!(e1 <= E_MAX)) bad = true;
         if (e1 > tol_e) more = true;
         E[i * ld + j] = e;
+        E[j * ld + i] = h;
       }
     if (__syncthreads_or(bad)) return -1;
     // X ← X + X E, into Y

@@ -30,12 +30,12 @@ def hermitian(rng, lam):
     return 0.5 * (a + a.conj().T)
 
 
-def check(G, S, m, got):
+def check(G, S, m, got, tol=1e-12):
     lam, C, rank = got
     assert rank == len(G)
     assert np.all(np.diff(lam) >= 0)
-    assert np.max(np.abs(C.conj().T @ G @ C - np.eye(m))) < 1e-12
-    assert np.linalg.norm(S @ C - (G @ C) * lam) < 1e-12 * np.linalg.norm(S)
+    assert np.max(np.abs(C.conj().T @ G @ C - np.eye(m))) < tol
+    assert np.linalg.norm(S @ C - (G @ C) * lam) < tol * np.linalg.norm(S)
 
 
 @pytest.mark.parametrize("n,m", SIZES)
@@ -64,6 +64,42 @@ def test_non_finite_projections_have_an_order(omb, n, m):
     lam, _, _ = rayleigh_ritz(G, np.full((n, n), np.nan), m)
     assert np.all(np.isnan(lam))
     check(G, S, m, rayleigh_ritz(G, S, m))
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("n,m", SIZES)
+def test_pairs_of_graded_matrices(omb, n, m, prec):
+    """Well-separated pairs, the refinement's ordinary case: eigenvalues from 0.3 to 300, G of condition
+    number 100.  (The FP32 tolerances stop the refinement earlier: at |E| ≤ 1e-6, so errors of ≈1e-12·n.)"""
+    from omb200.ops import rayleigh_ritz
+    rng = np.random.default_rng(100 + n)
+    G = hermitian(rng, np.geomspace(0.1, 10, n))
+    L = np.linalg.cholesky(G)
+    T = hermitian(rng, np.geomspace(0.3, 300, n))
+    S = L @ T @ L.conj().T
+    S = 0.5 * (S + S.conj().T)
+    lam, C, rank = got = rayleigh_ritz(G, S, m, precision=prec)
+    check(G, S, m, got, tol=1e-12 if prec == "fp64" else 1e-10)
+    assert np.allclose(lam, np.geomspace(0.3, 300, n)[:m], rtol=0, atol=1e-12 * 300 if prec == "fp64" else 1e-10 * 300)
+
+
+@pytest.mark.parametrize("gap", [0.0, 1e-14, 1e-11, 1e-8, 1e-5])
+@pytest.mark.parametrize("n,m", [s for s in SIZES if s[1] >= 2])
+def test_close_wanted_pairs(omb, n, m, gap):
+    """Two (then all) wanted eigenvalues `gap` apart: too close for the first-order refinement of the FP32
+    sweeps, so the FP64 Jacobi takes over; the pairs are as accurate as separated ones."""
+    from omb200.ops import rayleigh_ritz
+    rng = np.random.default_rng(200 + n)
+    for close in (2, m):
+        lam = np.linspace(1.0, 30.0, n)
+        lam[:close] = 0.4 + gap * np.arange(close)
+        G = hermitian(rng, np.linspace(1, 10, n))
+        L = np.linalg.cholesky(G)
+        S = L @ hermitian(rng, lam) @ L.conj().T
+        S = 0.5 * (S + S.conj().T)
+        got = rayleigh_ritz(G, S, m)
+        check(G, S, m, got)
+        assert np.allclose(got[0], lam[:m], rtol=0, atol=1e-12 * 30)
 
 
 def test_overflowing_operator_is_an_error(omb):
