@@ -490,7 +490,13 @@ __device__ __forceinline__ void finish(TrackState& s, int status) {
   s.op_ncol = 0; s.pw_ncol = 0; s.hmkh_ncol = 0;
 }
 
-constexpr int REFRESH = 8;  // iterations without a better residual after which AX and AP are recomputed
+// Iterations without a better residual after which a track starts again from X.  Plateaus of ordinary
+// solves last up to ≈10, and restarts there cost the conjugate directions: at 8 the 99th percentile of a
+// sweep's iterations went from 223 to 232 and a solve with the MPB preconditioner from 1346 to 1599
+// iterations; at 16 they are 222 and 1214.  At 24 the hard starts (two bands 4.5e-6 apart) take up to 946
+// iterations, at 16 up to 786 (at 12, 417).
+constexpr int REFRESH = 16;
+constexpr double BROKEN = 1e3;  // ratio of a residual to the best one that starts it again at once
 
 // The decisions after an update, for one track (one thread): residual norms from the sums `ra` of
 // k_update, locking, the phase's exits, and whether a Newton step
@@ -511,7 +517,10 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
   const int need = s.need;
   double maxres = 0;
   for (int i = 0; i < need; ++i) maxres = fmax(maxres, s.resid[i]);
-  if (maxres < 0.9 * s.resid_best) { s.resid_best = maxres; s.stall = 0; } else { s.stall++; }
+  // (a residual this far above the best one says that AX no longer belongs to X, or that a band came up
+  // that the block had missed)
+  const bool broken = maxres > BROKEN * s.resid_best;
+  if (maxres < 0.9 * s.resid_best || broken) { s.resid_best = maxres; s.stall = 0; } else { s.stall++; }
   while (s.nlocked < need && s.resid[s.nlocked] < prm.lock_tol) s.nlocked++;
   const bool last = prm.last_phase != 0;
   s.hmkh_ncol = 0;
@@ -555,11 +564,10 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
   // AX and AP are carried by their recurrences, whose rounding error grows where W and P are nearly
   // parallel: residuals that rise steadily (from ≈1e-11 in FP64), Ritz values below the spectrum, or a
   // zigzag on the few directions that the Gram floor leaves.  A track that has not improved for REFRESH
-  // iterations, or has a Ritz value that a positive operator cannot have, starts again from X: AX and AW
-  // formed afresh, no P, all columns unlocked.  (A pending Newton step recomputes them anyway, but takes
-  // no Ritz value from a broken block.  Of 360 starts of a 128² cell with two bands 4.5e-6 apart in k, 6
-  // stayed unconverged with P kept and none without.)
-  const bool broken = s.lam[0] <= 0.0;
+  // iterations, or whose residual jumped, starts again from X: AX and AW formed afresh, no P, all columns
+  // unlocked.  (A pending Newton step recomputes them anyway, but takes no Ritz value from a broken block.
+  // Of 360 starts of a 128² cell with two bands 4.5e-6 apart in k, 6 stayed unconverged with P kept and
+  // none without.)
   if (broken) s.hmkh_ncol = 0;
   if (broken || (s.hmkh_ncol == 0 && s.stall > 0 && s.stall % REFRESH == 0)) {
     s.nlocked = 0;
