@@ -16,8 +16,8 @@
 // Newton on k (reference: the per-band loop of ME/src/solve.jl:77-115 and
 // ME/src/solvers/gpu.jl:222-237): instead of converging a full eigensolve at every k, a
 // Newton step k ← k − (λ_b − ω²)/(2⟨x_b|∂M̂/∂k|x_b⟩) is taken inside the iteration as soon
-// as the Ritz value of band b is trustworthy; after a step AX is recomputed at the new k
-// and P is dropped.  The final step is only taken from an eigenpair converged to the
+// as the Ritz value of band b is trustworthy; after a step AX, AW and AP are recomputed at the
+// new k.  The final step is only taken from an eigenpair converged to the
 // tolerance, and the track stops when that step is below k_tol (the returned k is the
 // updated one, as in gpu.jl).  OUTER mode reproduces the reference loop exactly: a step
 // only after all block columns converged.
@@ -358,9 +358,9 @@ __global__ void __launch_bounds__(GramCfg<T>::NT, 1)
   // two-sum (Knuth) once the thread has summed GRAM_FOLD_ROWS rows (or a whole tile's share,
   // when that is more), so the rounding error of the track's sum stays at the FP32 level of
   // that many rows instead of growing with the number of tiles; FP64 sums directly.  Folding
-  // by rows rather than every tile keeps the fold (32 two-sums, the compensation terms in
-  // local memory) off the tiles of narrow tracks, whose items are split over ≈240 threads
-  // with one or two rows each.
+  // by rows rather than every tile keeps the fold (36 two-sums, the compensation terms in
+  // local memory) off the tiles of narrow tracks, whose items are split over up to 160 threads
+  // (n = 6) with one or two rows each.
   constexpr bool COMP = sizeof(T) == 4;
   constexpr int GRAM_FOLD_ROWS = 16;
   C acc[GRAM_E], lo[COMP ? GRAM_E : 1], t[COMP ? GRAM_E : 1];
@@ -596,7 +596,8 @@ template <typename T, int MB> struct UpdCfg {
   // rows per tile = consumer threads.  FP32: 15 consumer warps in one CTA per SM (16 warps, 128
   // registers).  FP64: 7 consumer warps; with the producer 8 warps, which leaves a thread 255 registers
   // in one CTA per SM (blocks of 7 and 9 columns: 86.9 → 86.2 and 167.0 → 164.4 ms for a solve of a 512×256
-  // slot row, against 8 consumer warps whose 168 registers spill) and 128 in two.  Blocks of up to 6
+  // slot row, against 8 consumer warps at 168 registers, whose body for 12 columns spilled 2.7 KB; it spills
+  // 32 bytes now) and 128 in two (the bodies for 5 and 6 columns spill 36 and 284 bytes).  Blocks of up to 6
   // columns run two CTAs, so that one tile's stores (half of its bytes) overlap the other's loads and
   // products: the sweep of twelve 256² instances 292.3 → 275.7 ms, a 512² solve 89.9 → 86.6, against one
   // CTA of 256 rows (two CTAs of 128, 160 and 192 rows: 0.99, 1.04 and 1.05–1.06 of its speed on the sweep).
