@@ -519,7 +519,7 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
   for (int i = 0; i < need; ++i) maxres = fmax(maxres, s.resid[i]);
   // (a residual this far above the best one says that AX no longer belongs to X, or that a band came up
   // that the block had missed)
-  const bool broken = maxres > BROKEN * s.resid_best;
+  const bool broken = maxres > prm.tol && maxres > BROKEN * s.resid_best;
   if (maxres < 0.9 * s.resid_best || broken) { s.resid_best = maxres; s.stall = 0; } else { s.stall++; }
   while (s.nlocked < need && s.resid[s.nlocked] < prm.lock_tol) s.nlocked++;
   const bool last = prm.last_phase != 0;
