@@ -494,8 +494,10 @@ __device__ __forceinline__ void finish(TrackState& s, int status) {
 // solves last up to ≈10, and restarts there cost the conjugate directions: at 8 the 99th percentile of a
 // sweep's iterations went from 223 to 232 and a solve with the MPB preconditioner from 1346 to 1599
 // iterations; at 16 they are 222 and 1214.  At 24 the hard starts (two bands 4.5e-6 apart) take up to 946
-// iterations, at 16 up to 786 (at 12, 417).
-constexpr int REFRESH = 16;
+// iterations, at 16 up to 786 (at 12, 417).  The reference loop's blocks have no guard column and wait for
+// their slowest one, on plateaus of tens of iterations: of 78 such FP64 solves at 3e-12 17 ended at the
+// iteration limit without restarts, 11 (one of them new) with 16 and 9 (none new) with 64.
+constexpr int REFRESH = 16, REFRESH_OUTER = 64;
 constexpr double BROKEN = 1e3;  // ratio of a residual to the best one that starts it again at once
 
 // The decisions after an update, for one track (one thread): residual norms from the sums `ra` of
@@ -564,12 +566,12 @@ __device__ inline void control_track(TrackState& s, const double* ra, const Iter
   // AX and AP are carried by their recurrences, whose rounding error grows where W and P are nearly
   // parallel: residuals that rise steadily (from ≈1e-11 in FP64), Ritz values below the spectrum, or a
   // zigzag on the few directions that the Gram floor leaves.  A track that has not improved for REFRESH
-  // iterations, or whose residual jumped, starts again from X: AX and AW formed afresh, no P, all columns
+  // iterations (REFRESH_OUTER in the reference loop), or whose residual jumped, starts again from X: AX and AW formed afresh, no P, all columns
   // unlocked.  (A pending Newton step recomputes them anyway, but takes no Ritz value from a broken block.
   // Of 360 starts of a 128² cell with two bands 4.5e-6 apart in k, 6 stayed unconverged with P kept and
   // none without.)
   if (broken) s.hmkh_ncol = 0;
-  if (broken || (s.hmkh_ncol == 0 && s.stall > 0 && s.stall % REFRESH == 0)) {
+  if (broken || (s.hmkh_ncol == 0 && s.stall > 0 && s.stall % (s.mode == MODE_NEWTON_OUTER ? REFRESH_OUTER : REFRESH) == 0)) {
     s.nlocked = 0;
     s.nWa = M;
     s.nP = 0;
